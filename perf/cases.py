@@ -13,6 +13,7 @@ N(0, 0.1): the distributions of the benchmark's configurations.
 
 import math
 
+import numpy as np
 import torch
 
 from onnx_light_cpu_b200 import MatMulNBitsSession, MatMulNBitsWeights, register_kernels
@@ -156,19 +157,25 @@ def _host(tensor):
     return None if tensor is None else tensor.cpu().numpy()
 
 
-def prepare(case, seed):
+def _drawn(case, seed):
+    """Operands by node, activations by stage."""
     gen = torch.Generator(device=DEVICE)
     gen.manual_seed(seed)
-    m, kind = case["m"], case["kind"]
     operands = {name: _Operands(case, k, n, gen) for name, k, n in _shapes(case)}
+    stages = STAGES if case["kind"] == "layer" else (("node", ("node",)),)
+    inputs = {stage: torch.randn(case["m"], operands[names[0]].k, device=DEVICE, generator=gen) for stage, names in stages}
+    return operands, inputs
+
+
+def prepare(case, seed):
+    m, kind = case["m"], case["kind"]
+    operands, inputs = _drawn(case, seed)
     torch.cuda.synchronize()  # the weights are in place before a handle lays out what it derives from them
     if kind == "layer":
         layer = DecoderLayerProjections(operands)
-        inputs = {stage: torch.randn(m, operands[names[0]].k, device=DEVICE, generator=gen) for stage, names in STAGES}
         layer.outputs(m)
         return {"case": case, "layer": layer, "inputs": inputs}
-    node = operands["node"]
-    a = torch.randn(m, node.k, device=DEVICE, generator=gen)
+    node, a = operands["node"], inputs["node"]
     options = {"K": node.k, "N": node.n, "bits": node.bits, "block_size": node.block_size}
     if kind == "operator":
         session = MatMulNBitsSession(_host(node.b), _host(node.scales), _host(node.zero_points), _host(node.bias),
@@ -186,3 +193,40 @@ def run(state):
         return state["session"].run(state["a"])
     state["weights"].matmul_device(state["a"], state["y"], accuracy_level=case["level"])
     return state["y"]
+
+
+def _product64(case, operand, a):
+    """Y of one node in 64 bits. At level 4 the activations are first the operator's int8 codes, one scale per block."""
+    m, k, n, bits, block = case["m"], operand.k, operand.n, operand.bits, operand.block_size
+    blocks = k // block
+    if case["level"] == 4:
+        groups = a.cpu().numpy().reshape(m, blocks, block)  # on the host: the codes follow from IEEE single divisions
+        scale = np.abs(groups).max(axis=2, keepdims=True) / np.float32(127.0)
+        codes = np.rint(groups / scale).clip(-127.0, 127.0)
+        a = torch.from_numpy(codes.astype(np.float64) * scale.astype(np.float64)).to(DEVICE).reshape(m, k)
+    a = a.double()
+    y = torch.empty(m, n, dtype=torch.float64, device=DEVICE)
+    rows = max(1, (1 << 27) // k)  # columns of Y at a time: about 1 GB of weights in 64 bits
+    for first in range(0, n, rows):
+        codes = operand.b[first:first + rows].flatten(1)
+        if bits == 4:
+            codes = torch.stack((codes & 15, codes >> 4), dim=2)
+        codes = codes.reshape(-1, blocks, block).double()
+        zero = torch.full((codes.shape[0], blocks), float(1 << (bits - 1)), dtype=torch.float64, device=DEVICE)
+        if operand.zero_points is not None:
+            zero = operand.zero_points[first:first + rows]
+            if bits == 4:
+                zero = torch.stack((zero & 15, zero >> 4), dim=2).flatten(1)[:, :blocks]
+            zero = zero.double()
+        scale = operand.scales.view(n, blocks)[first:first + rows].double()
+        y[:, first:first + rows] = a @ ((codes - zero[:, :, None]) * scale[:, :, None]).flatten(1).t()
+    if operand.bias is not None:
+        y += operand.bias.double()
+    return y
+
+
+def exact(case, seed):
+    operands, inputs = _drawn(case, seed)
+    if case["kind"] == "layer":
+        return {name: _product64(case, operands[name], inputs[stage]) for stage, names in STAGES for name in names}
+    return _product64(case, operands["node"], inputs["node"])
