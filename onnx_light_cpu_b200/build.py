@@ -30,6 +30,7 @@ CUDA_SOURCES = [
     "csrc/nbits_int8.cu",
     "csrc/nbits_int8_mma.cu",
     "csrc/nbits_gemm_tcgen05.cu",
+    "csrc/nbits_gemm_i8_tcgen05.cu",
 ]
 CUDA_HEADERS = ["csrc/nbits_common.cuh", "csrc/nbits_digits.cuh", "csrc/nbits_ptx.cuh", "csrc/nbits_tma.cuh", "csrc/nbits_mma_common.cuh",
                 "../include/matmulnbits_b200.h"]

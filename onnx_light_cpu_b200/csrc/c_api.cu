@@ -315,6 +315,19 @@ bool DigitSlicesWanted(const WeightView &w, std::int64_t m) {
   return m >= 5 || (m >= 3 && w.k >= 8192);
 }
 
+// accuracy_level 4: whether AUTO sends the call to the tcgen05 integer GEMM. 8-bit weights always (K = N = 4096, blocks of
+// 128, M = 17 / 128: 63 / 372 us on dp4a, 14 / 23 there). 4-bit nodes that the sixteen-token kernel takes stay with it
+// for two passes (M = 17 ... 32, block 32: 19-21 us on both at N = 4096, 32 against 35 at N = 14336; M = 33: 23 against
+// 21 and 45 against 45; M = 64: 30 against 22, 59 against 45) and small nodes for four (K = N = 1024, M = 33 / 64: 12 / 13
+// against 13.3; M = 128: 17 against 13).
+bool GemmI8Preferred(const WeightView &w, std::int64_t m) {
+  if (!mnb::GemmI8Supports(w, m)) {
+    return false;
+  }
+  const bool few = m <= 32 || (m <= 64 && w.n * w.k <= (std::int64_t{2} << 20));
+  return !(few && w.bits == 4 && mnb::Int8MmaScratchBytes(w, m) != 0);
+}
+
 // Core dispatch. The caller holds h->mutex and has made h->device current.
 int Dispatch(mnb_weights *h, const float *a_dev, std::int64_t m, int accuracy_level, int path,
              OutputView out, cudaStream_t stream) {
@@ -567,6 +580,18 @@ int Dispatch(mnb_weights *h, const float *a_dev, std::int64_t m, int accuracy_le
     break;
   }
   case MNB_PATH_INT8_MMA: {
+    if (path == MNB_PATH_AUTO && GemmI8Preferred(w, m)) {
+      const int rc = Grow(&h->scratch_a, &h->scratch_a_bytes, mnb::GemmI8ScratchBytes(w, m, h->sm_count));
+      if (rc != MNB_OK) {
+        return rc;
+      }
+      name = mnb::LaunchGemmI8(&w, &out, 1, a_dev, m, static_cast<unsigned char *>(h->scratch_a), h->status_dev, stream,
+                               h->sm_count);
+      if (name != nullptr) {
+        break;
+      }
+      cudaGetLastError();
+    }
     const std::size_t need = mnb::Int8MmaScratchBytes(w, m);
     if (need != 0) {
       const int rc = Grow(&h->scratch_a, &h->scratch_a_bytes, need);
@@ -921,8 +946,29 @@ int mnb_matmul_device_group(mnb_weights *const *handles, int count, const float 
     // one launch: the nodes' tiles form one sequence behind activations staged once
     name = mnb::LaunchDecodeResidentGroup(nodes, outs, count, a_dev, m, first->status_dev, s, first->sm_count);
   } else if (accuracy_level == 4 && count > 1) {
-    // activations quantized once, then one integer-MMA launch per node
+    // activations quantized once, then a tcgen05 product per node or one integer-MMA launch for all of them
     std::size_t need = 0;
+    for (int i = 0; i < count; ++i) {
+      const std::size_t bytes = GemmI8Preferred(nodes[i], m) ? mnb::GemmI8ScratchBytes(nodes[i], m, first->sm_count) : 0;
+      need = bytes == 0 ? 0 : (bytes > need ? bytes : need);
+      if (bytes == 0) {
+        break;
+      }
+    }
+    if (need != 0) {
+      const int rc = Grow(&first->scratch_a, &first->scratch_a_bytes, need);
+      if (rc != MNB_OK) {
+        return rc;
+      }
+      name = mnb::LaunchGemmI8(nodes, outs, count, a_dev, m, static_cast<unsigned char *>(first->scratch_a),
+                               first->status_dev, s, first->sm_count);
+      if (name != nullptr) {
+        mnb::t_last_kernel = name;
+        return MNB_OK;
+      }
+      cudaGetLastError();
+    }
+    need = 0;
     for (int i = 0; i < count; ++i) {
       const std::size_t bytes = mnb::Int8MmaScratchBytes(nodes[i], m);
       need = bytes == 0 ? 0 : (bytes > need ? bytes : need);

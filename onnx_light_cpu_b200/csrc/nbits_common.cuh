@@ -322,6 +322,17 @@ const char *LaunchGemmTcgen05(const WeightView &w, const float *a, std::int64_t 
 std::size_t GemmTcgen05ScratchBytes(const WeightView &w, std::int64_t m, int sm_count);
 bool GemmTcgen05Supports(const WeightView &w, std::int64_t m);
 
+// Y = part 0 + part 1 + ... (in that order) + bias of a product whose K was shared: partial [parts][m][n].
+bool LaunchSplitKSum(const float *partial, int parts, std::int64_t m, const WeightView &w, OutputView out,
+                     cudaStream_t stream, int sms);
+
+// accuracy_level 4, more than sixteen tokens: exact block dots on tcgen05. Sibling nodes (same K, bits and block
+// size) share the quantized activations. `scratch`: the most that GemmI8ScratchBytes says of any of them.
+bool GemmI8Supports(const WeightView &w, std::int64_t m);
+std::size_t GemmI8ScratchBytes(const WeightView &w, std::int64_t m, int sm_count);
+const char *LaunchGemmI8(const WeightView *nodes, const OutputView *outs, int count, const float *a, std::int64_t m,
+                         unsigned char *scratch, int *status_word, cudaStream_t stream, int sm_count);
+
 // accuracy_level 4.
 const char *LaunchQuantizeA(const float *a, std::int64_t m, std::int64_t k, int block_size,
                             std::int8_t *aq, float *a_scales, cudaStream_t stream);

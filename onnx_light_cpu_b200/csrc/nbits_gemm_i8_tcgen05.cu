@@ -1,0 +1,1011 @@
+// accuracy_level 4 with many tokens for sm_100a: integer GEMM on tcgen05 (kind::i8) whose accumulators
+// restart with every quantization block.
+//
+//     Y[m, n] = sum_b sa[m, b] * scale[n, b] * dot_b[m, n],   dot_b = sum over block b of aq * (q - zp)
+//
+// The tensor core computes the exact int32 dots of one block for a tile of 128 weight rows (TMEM lanes) x BT
+// tokens (TMEM columns); the epilogue warps scale and add them in fp32 while the next blocks are multiplied.
+//
+// What bounds it: the scaling. Every output of every block is a conversion, a product of the two scales and a
+// multiply-add on the ordinary pipes (M N K / block of each, 8 MMA issue slots of int8 against several hundred cycles
+// of scaling per 128 x 128 x 32), and the hand-overs around it: removing the arithmetic alone leaves 60 of the 79 us
+// of M = 512, N = K = 4096, blocks of 32, removing TMEM loads, MMAs and unpacking as well 31. So int8 operands (half the
+// shared-memory traffic of bf16 ones), weights turned into signed bytes q - zp in seven instructions per eight codes,
+// and two scaling warpgroups that take turns.
+//
+// Per CTA, 512 threads, a tile of 128 weight rows x BT tokens in two halves of BT / 2 tokens:
+//   warp 0       TMA producer: per 128-k step the activation codes (128-byte swizzle) and the packed weight rows,
+//                and the activation scales of the step's blocks
+//   warps 1, 2   MMA issuers, one lane and one half of the tokens each, round by round into the half's TMEM
+//   warp 3       the weight scales of the 128 rows into shared memory, four blocks at a time
+//   warps 4..7   4-bit weights: packed nibbles to signed bytes q - zp in the swizzled tile the MMA reads. 8-bit
+//                codes enter as unsigned bytes straight from the TMA copy; their zero points leave through
+//                dot - zp * (sum of the activation codes), exact in fp32 below 2^24
+//   warps 8..15  scaling, a warpgroup per half. tcgen05.ld 16x256b gives a lane four rows and a quarter of the columns,
+//                so a pair of token scales is one 8-byte shared-memory read per four rows (the 32x32b form, one row
+//                a lane, reads every token scale in every lane)
+// A lane adds up sixteen blocks before it adds their sum to its total (in shared memory): one running sum over
+// all blocks of a long row rounds three times as much.
+// Registers are moved from the first two warpgroups (64 a thread) to the scaling ones (192).
+//
+// Measured (call with its quantization, us; before: the sixteen-token kernel in passes, dp4a for 8-bit weights), K = 4096:
+//   M = 512, N = 4096, blocks of 32    186 -> 79      M = 64, N = 4096, 8-bit blocks of 32    204 -> 24
+//   M = 128, N = 14336, blocks of 32   111 -> 78      M = 128, N = 14336, 8-bit blocks of 128 963 -> 39
+// All barrier waits are bounded; on a timeout the status word is set and the CTA drains to its tear-down.
+
+#include "nbits_common.cuh"
+#include "nbits_ptx.cuh"
+#include "nbits_tma.cuh"
+
+#include <cstdint>
+
+namespace mnb {
+namespace {
+
+constexpr int kRows = 128;      // weight rows per CTA (TMEM lanes)
+constexpr int kStepK = 128;     // k per pipeline stage: one 128-byte swizzle atom of int8
+constexpr int kSlabK = 32;      // k per MMA
+constexpr int kStages = 3;      // TMA ring
+constexpr int kBuffers = 3;     // dequantized weight tiles (4-bit)
+constexpr int kScaleSlots = 4;  // activation scales, one slot per step (or per block, where blocks are longer)
+constexpr int kWeightSlots = 4; // weight scales of the 128 rows, four blocks a slot
+constexpr int kMaxEntries = 4;  // blocks per slot: 128 / 32
+constexpr int kDequantWarps = 4;
+constexpr int kScaleWarps = 8;
+constexpr int kThreads = 256 + kScaleWarps * 32;
+constexpr int kFlushBlocks = 16;
+constexpr int kLowRegs = 64;    // registers a thread after the move: 256 x 64 + 256 x 192 = 512 x 128
+constexpr int kHighRegs = 192;
+// What a slab of constant bytes on both sides adds to every dot of 4-bit weights: above the largest |dot| of a block
+// of 256 (15 * 127 * 256), so that every accumulator is a non-negative integer below 2^20.
+constexpr int kBiasByte = 127;
+constexpr int kBias = kBiasByte * kBiasByte * kSlabK;
+constexpr int kBiasBytes = kRows * kSlabK;
+
+template <int BT, int BITS> struct I8Smem {
+  static constexpr int kRowP = kStepK * BITS / 8;                 // packed bytes of a row per step: 64 / 128
+  static constexpr int kStageA = BT * kStepK;
+  static constexpr int kStageP = kRows * kRowP;                   // 4-bit: packed; 8-bit: the MMA's own tile
+  static constexpr int kBufferW = BITS == 4 ? kRows * kStepK : 0;
+  static constexpr int kSums = BITS == 8 ? 2 : 1;                 // scales, and for 8-bit weights code sums
+  static constexpr int kSlot = kMaxEntries * BT * 4 * kSums;
+  static constexpr int kWeightSlot = kRows * 16 * kSums;          // [rows][4 blocks], 8-bit: zero points behind them
+  static constexpr int kSumBytes = kRows * BT * 4;                // totals of the scaling warps
+  static constexpr int kTotal =
+      kStages * (kStageA + kStageP) + kBuffers * kBufferW + kScaleSlots * kSlot + kWeightSlots * kWeightSlot +
+      kSumBytes + kBiasBytes + 512 + 1024;
+};
+
+struct I8Params {
+  WeightView w;
+  OutputView out;
+  int m_total;
+  int *status;
+  std::uint32_t idesc;
+  int vector_scales;     // the scales of two (four) consecutive blocks of a row lie aligned
+  float *partial;        // K shared between CTAs: [parts][m_total][n], summed by a kernel behind this one
+};
+
+// Quantization of the activations, one thread per eight k: per (token, block) sa = max|A| / 127 and the codes
+// clamp(rint(A / sa), -127, 127), IEEE single divisions as everywhere at this level. A block with a NaN or an
+// infinity gets scale NaN and codes 0. PERMUTE stores the eight codes as k 0,2,4,6,1,3,5,7, the order in which
+// the packed nibbles come out; otherwise (8-bit weights) the table holds, behind the scales of each block, the sums
+// of its codes.
+template <bool PERMUTE>
+__global__ void __launch_bounds__(256)
+    nbits_quantize_a_i8_kernel(const float *a, int m, std::int64_t k, int k_pad, int block_size, int m_pad,
+                               std::int8_t *aq, float *table) {
+  ptx::GridDependencyLaunch();
+  ptx::GridDependencyWait();
+  const int per_row = k_pad / 8;
+  const int group = block_size / 8; // lanes of a block: 4 .. 32, consecutive and aligned
+  const std::int64_t total = static_cast<std::int64_t>(m) * per_row;
+  const std::int64_t index = static_cast<std::int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  const bool live = index < total;
+  const int row = live ? static_cast<int>(index / per_row) : 0;
+  const int k0 = live ? static_cast<int>(index - static_cast<std::int64_t>(row) * per_row) * 8 : 0;
+  float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  if (live && k0 < k) {
+    const float4 *src = reinterpret_cast<const float4 *>(a + static_cast<std::int64_t>(row) * k + k0);
+    const float4 lo = __ldg(src);
+    const float4 hi = __ldg(src + 1);
+    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+    v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+  }
+  float amax = 0.0f;
+  bool bad = false;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float x = fabsf(v[i]);
+    amax = fmaxf(amax, x);
+    bad = bad || !(x <= 3.4028235e38f);
+  }
+  int flag = bad ? 1 : 0;
+  for (int offset = 1; offset < group; offset <<= 1) {
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
+    flag |= __shfl_xor_sync(0xffffffffu, flag, offset);
+  }
+  const float sa = flag != 0 ? __int_as_float(0x7fc00000) : __fdiv_rn(amax, 127.0f);
+  int q[8];
+  int sum = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    q[i] = 0;
+    if (sa > 0.0f) {
+      q[i] = static_cast<int>(fminf(127.0f, fmaxf(-127.0f, rintf(__fdiv_rn(v[i], sa)))));
+    }
+    sum += q[i];
+  }
+  for (int offset = 1; offset < group; offset <<= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+  }
+  if (!live) {
+    return;
+  }
+  auto pack = [&](int i0, int i1, int i2, int i3) {
+    return static_cast<std::uint32_t>(q[i0] & 0xff) | (static_cast<std::uint32_t>(q[i1] & 0xff) << 8) |
+           (static_cast<std::uint32_t>(q[i2] & 0xff) << 16) | (static_cast<std::uint32_t>(q[i3] & 0xff) << 24);
+  };
+  uint2 packed;
+  packed.x = PERMUTE ? pack(0, 2, 4, 6) : pack(0, 1, 2, 3);
+  packed.y = PERMUTE ? pack(1, 3, 5, 7) : pack(4, 5, 6, 7);
+  *reinterpret_cast<uint2 *>(aq + static_cast<std::int64_t>(row) * k_pad + k0) = packed;
+  if (k0 % block_size == 0) {
+    const std::int64_t block = k0 / block_size;
+    if (PERMUTE) {
+      table[block * m_pad + row] = sa;
+    } else {
+      table[2 * block * m_pad + row] = sa;
+      table[(2 * block + 1) * m_pad + row] = static_cast<float>(sum); // at most 127 * 256: exact
+    }
+  }
+}
+
+__device__ __forceinline__ std::uint64_t Pair(float lo, float hi) {
+  std::uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 Unpair(std::uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ std::uint64_t Mul2(std::uint64_t a, std::uint64_t b) {
+  std::uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ std::uint64_t Fma2(std::uint64_t a, std::uint64_t b, std::uint64_t c) {
+  std::uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// 16 lanes x 8 * (R / 4) columns: lane t receives rows t / 4 (registers 4 i, 4 i + 1) and t / 4 + 8 (4 i + 2,
+// 4 i + 3) of columns 8 i + 2 (t % 4) and the next one.
+__device__ __forceinline__ void TmemLoadRows(std::uint32_t taddr, std::uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+               "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                 "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                 "=r"(v[15])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void TmemLoadRows(std::uint32_t taddr, std::uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+
+
+// Waits for the lane's loads; the registers pass through it, so that no use of them can move in front of it.
+__device__ __forceinline__ void TmemWaitRows(std::uint32_t (&v)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]),
+                 "+r"(v[15])
+               :
+               : "memory");
+}
+__device__ __forceinline__ void TmemWaitRows(std::uint32_t (&v)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+               :
+               : "memory");
+}
+
+// D[tmem] (+)= A[smem desc] * B[smem desc], 8-bit integers -> int32. One thread issues.
+__device__ __forceinline__ void UmmaI8(std::uint32_t tmem_d, std::uint64_t desc_a, std::uint64_t desc_b,
+                                       std::uint32_t idesc, std::uint32_t accumulate) {
+  asm volatile("{\n\t"
+               ".reg .pred p;\n\t"
+               "setp.ne.b32 p, %4, 0;\n\t"
+               "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
+               "}" ::"r"(tmem_d),
+               "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+               : "memory");
+}
+
+// 1, 2 or 4 consecutive floats of shared memory, aligned to their number.
+__device__ __forceinline__ void LoadRun(const float *p, float (&v)[1]) { v[0] = *p; }
+__device__ __forceinline__ void LoadRun(const float *p, float (&v)[2]) {
+  const float2 f = *reinterpret_cast<const float2 *>(p);
+  v[0] = f.x; v[1] = f.y;
+}
+__device__ __forceinline__ void LoadRun(const float *p, float (&v)[4]) {
+  const float4 f = *reinterpret_cast<const float4 *>(p);
+  v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+}
+
+// Four codes in the low nibbles of `q` as signed bytes q - zp (`zps` = zp in every byte): the bias of 0x80 keeps
+// the bytes from borrowing from one another, and taking it out again by XOR leaves two's complement.
+__device__ __forceinline__ std::uint32_t SignedCodes(std::uint32_t q, std::uint32_t zps) {
+  return (((q & 0x0f0f0f0fu) | 0x80808080u) - zps) ^ 0x80808080u;
+}
+
+// SPB: slabs (MMAs) of a block: block size / 32. The tokens of the tile are two halves with an issuing lane, a half of
+// the TMEM and a scaling warpgroup each: while one warpgroup meets its barriers the other one scales. A round is what an issuer hands to its
+// warpgroup at once: the blocks of a 128-k step, or one longer block.
+template <int BT, int BITS, int SPB>
+__global__ void __launch_bounds__(kThreads, 1)
+    nbits_gemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
+                                 const __grid_constant__ CUtensorMap map_p,
+                                 const __grid_constant__ CUtensorMap map_s, const I8Params p) {
+  using Smem = I8Smem<BT, BITS>;
+  constexpr int kDotBuffers = BT == 128 ? 4 : 8;                         // TMEM accumulators of BT columns
+  constexpr int kHalf = BT / 2;                                          // tokens of a half
+  constexpr int kRoundBlocks = SPB < 4 ? 4 / SPB : 1;
+  constexpr int kRoundSlabs = kRoundBlocks * SPB;
+  constexpr int kRoundBuffers = kDotBuffers / kRoundBlocks;
+  constexpr bool kBiased = BITS == 4;
+  constexpr int kSlabs = kStepK / kSlabK;                                // slabs per step
+  constexpr int kEntries = SPB < kSlabs ? kSlabs / SPB : 1;              // blocks per scale slot
+  constexpr int kSlotSteps = SPB > kSlabs ? SPB / kSlabs : 1;            // steps per scale slot
+  extern __shared__ __align__(1024) unsigned char smem_dyn[];
+  unsigned char *smem = smem_dyn + ((1024u - (ptx::SmemAddr(smem_dyn) & 1023u)) & 1023u);
+  unsigned char *ring_a = smem;
+  unsigned char *ring_p = ring_a + kStages * Smem::kStageA;
+  unsigned char *buf_w = ring_p + kStages * Smem::kStageP;
+  unsigned char *slots = buf_w + kBuffers * Smem::kBufferW;
+  unsigned char *weight_slots = slots + kScaleSlots * Smem::kSlot;
+  std::uint64_t *totals = reinterpret_cast<std::uint64_t *>(weight_slots + kWeightSlots * Smem::kWeightSlot);
+  unsigned char *bias_tile = reinterpret_cast<unsigned char *>(totals + Smem::kSumBytes / 8);
+  std::uint64_t *bars = reinterpret_cast<std::uint64_t *>(bias_tile + kBiasBytes);
+  std::uint64_t *full_tma = bars;                      // [stages] codes and packed weights landed
+  std::uint64_t *empty = full_tma + kStages;           // [stages] MMAs of the stage retired
+  std::uint64_t *w_full = empty + kStages;             // [buffers] weights as signed bytes
+  std::uint64_t *w_empty = w_full + kBuffers;          // [buffers] MMAs that read the buffer retired
+  std::uint64_t *d_full = w_empty + kBuffers;          // [2 halves][dot buffers] dots of a round complete
+  std::uint64_t *d_empty = d_full + 2 * kDotBuffers;   // [2 halves][dot buffers] read by the half's scaling warps
+  std::uint64_t *s_full = d_empty + 2 * kDotBuffers;   // [scale slots]
+  std::uint64_t *s_empty = s_full + kScaleSlots;
+  std::uint64_t *t_full = s_empty + kScaleSlots;       // [weight scale slots]
+  std::uint64_t *t_empty = t_full + kWeightSlots;
+  std::uint32_t *tmem_slot = reinterpret_cast<std::uint32_t *>(t_empty + kWeightSlots);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  constexpr std::uint32_t kTmemColumns = BT * kDotBuffers < 32 ? 32 : BT * kDotBuffers;
+
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5;
+  const int lane = tid & 31;
+  const int n0 = blockIdx.x * kRows;
+  const int m0 = blockIdx.y * BT;
+  ptx::GridDependencyLaunch();
+
+  // this CTA's part of K: whole scale slots
+  const int parts = static_cast<int>(gridDim.z);
+  const int part = static_cast<int>(blockIdx.z);
+  const int slots_total = (p.w.n_blocks + kEntries - 1) / kEntries;
+  const int slot_begin = static_cast<int>(static_cast<std::int64_t>(part) * slots_total / parts);
+  const int slot_end = static_cast<int>(static_cast<std::int64_t>(part + 1) * slots_total / parts);
+  const int step0 = slot_begin * kSlotSteps;
+  const int steps = (slot_end - slot_begin) * kSlotSteps;
+  // codes and scales are padded with zeros to whole slots, so the last one is multiplied like the others
+  const int b_begin = slot_begin * kEntries;
+  const int rounds = (slot_end - slot_begin) * kEntries / kRoundBlocks;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      ptx::MbarInit(&full_tma[s], 1);
+      ptx::MbarInit(&empty[s], 2);     // both issuers
+    }
+    for (int b = 0; b < kBuffers; ++b) {
+      ptx::MbarInit(&w_full[b], kDequantWarps);
+      ptx::MbarInit(&w_empty[b], 2);
+    }
+    for (int d = 0; d < 2 * kDotBuffers; ++d) {
+      ptx::MbarInit(&d_full[d], 1);
+      ptx::MbarInit(&d_empty[d], kScaleWarps / 2);
+    }
+    for (int q = 0; q < kScaleSlots; ++q) {
+      ptx::MbarInit(&s_full[q], 1);
+      ptx::MbarInit(&s_empty[q], kScaleWarps);
+    }
+    for (int q = 0; q < kWeightSlots; ++q) {
+      ptx::MbarInit(&t_full[q], 1);
+      ptx::MbarInit(&t_empty[q], kScaleWarps);
+    }
+    *abort_flag = 0;
+    ptx::FenceMbarInit();
+  }
+  if (warp == 0) {
+    ptx::TmemAlloc(tmem_slot, kTmemColumns);
+    ptx::TmemRelinquish();
+  }
+  if (kBiased && warp >= 8) {
+    *reinterpret_cast<uint4 *>(bias_tile + (tid - 256) * 16) =
+        make_uint4(kBiasByte * 0x01010101u, kBiasByte * 0x01010101u, kBiasByte * 0x01010101u, kBiasByte * 0x01010101u);
+    ptx::FenceProxyAsyncShared();
+  }
+  ptx::TcFenceBefore();
+  __syncthreads();
+  ptx::TcFenceAfter();
+  const std::uint32_t tmem_base = *tmem_slot;
+
+  if (warp < 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLowRegs));
+    if (warp == 0 && lane == 0) {
+      // ------------------------------- TMA producer -------------------------------
+      ptx::PrefetchTensorMap(&map_a);
+      ptx::PrefetchTensorMap(&map_p);
+      ptx::PrefetchTensorMap(&map_s);
+      // the weights are constant: the first ring of them is asked for while the quantization still runs
+      const int ahead = steps < kStages ? steps : kStages;
+      for (int ks = 0; ks < ahead; ++ks) {
+        ptx::MbarArriveExpectTx(&full_tma[ks], Smem::kStageA + Smem::kStageP);
+        ptx::TmaLoad2D(ring_p + ks * Smem::kStageP, &map_p, (step0 + ks) * Smem::kRowP, n0, &full_tma[ks]);
+      }
+      ptx::GridDependencyWait(); // codes and scales come from the kernel launched just before
+      int s = 0, q = 0;
+      std::uint32_t phase = 1, slot_phase = 1;
+#pragma unroll 1
+      for (int ks = 0; ks < steps; ++ks) {
+        if (!ptx::MbarWaitHot(&empty[s], phase)) {
+          ReportStatus(p.status, kDeviceTimeoutEmptyBarrier);
+          *abort_flag = 1;
+          break;
+        }
+        if (ks >= ahead) {
+          ptx::MbarArriveExpectTx(&full_tma[s], Smem::kStageA + Smem::kStageP);
+          ptx::TmaLoad2D(ring_p + s * Smem::kStageP, &map_p, (step0 + ks) * Smem::kRowP, n0, &full_tma[s]);
+        }
+        ptx::TmaLoad2D(ring_a + s * Smem::kStageA, &map_a, (step0 + ks) * kStepK, m0, &full_tma[s]);
+        if (kSlotSteps == 1 || (ks & (kSlotSteps - 1)) == 0) {
+          if (!ptx::MbarWaitHot(&s_empty[q], slot_phase)) {
+            ReportStatus(p.status, kDeviceTimeoutEmptyBarrier);
+            *abort_flag = 1;
+            break;
+          }
+          constexpr int kTableRows = kEntries * Smem::kSums;
+          ptx::MbarArriveExpectTx(&s_full[q], kTableRows * BT * 4);
+          ptx::TmaLoad2D(slots + q * Smem::kSlot, &map_s, m0, (slot_begin + ks / kSlotSteps) * kTableRows, &s_full[q]);
+          if (++q == kScaleSlots) {
+            q = 0;
+            slot_phase ^= 1u;
+          }
+        }
+        if (++s == kStages) {
+          s = 0;
+          phase ^= 1u;
+        }
+      }
+    } else if ((warp == 1 || warp == 2) && lane == 0) {
+      // ------------------------------- MMA issuer -------------------------------
+      // An issuing lane's own instruction stream was the bound of the first form (350 cycles per MMA with the slab,
+      // stage and buffer worked out for each): everything inside a step is known when the kernel is compiled.
+      const int half = warp - 1;
+      const std::uint64_t desc_a0 = ptx::UmmaDescKMajorSw128(ptx::SmemAddr(ring_a) + half * kHalf * kStepK);
+      const std::uint64_t desc_w0 = ptx::UmmaDescKMajorSw128(ptx::SmemAddr(BITS == 4 ? buf_w : ring_p));
+      // the constant slab: no swizzle, 8 x 16 byte cores 128 bytes apart along k and 256 along the rows
+      const std::uint64_t desc_bias = static_cast<std::uint64_t>((ptx::SmemAddr(bias_tile) & 0x3ffffu) >> 4) |
+                                      (static_cast<std::uint64_t>(128 >> 4) << 16) |
+                                      (static_cast<std::uint64_t>(256 >> 4) << 32) | (static_cast<std::uint64_t>(1) << 46);
+      const std::uint32_t tmem_half = tmem_base + half * kDotBuffers * kHalf;
+      std::uint64_t *full = d_full + half * kDotBuffers;
+      std::uint64_t *free = d_empty + half * kDotBuffers;
+      std::uint64_t *landed = BITS == 4 ? w_full : full_tma;
+      constexpr int kLanded = BITS == 4 ? kBuffers : kStages;
+      constexpr std::uint32_t kTileW = BITS == 4 ? Smem::kBufferW : Smem::kStageP;
+      int s = 0, w = 0, d = 0;
+      std::uint32_t w_phase = 0, d_phase = 1;
+      bool ok = true;
+#pragma unroll 1
+      for (int ks = 0; ks < steps; ++ks) {
+        if (!ptx::MbarWaitHot(&landed[w], w_phase)) {
+          ok = false;
+          break;
+        }
+        ptx::TcFenceAfter();
+        const std::uint64_t desc_a = desc_a0 + static_cast<std::uint32_t>(s * Smem::kStageA >> 4);
+        const std::uint64_t desc_w = desc_w0 + static_cast<std::uint32_t>(w * kTileW >> 4);
+        const bool opens = kRoundSlabs <= kSlabs || (ks & (kSlotSteps - 1)) == 0;   // a round begins with this step
+        const bool closes = kRoundSlabs <= kSlabs || (ks & (kSlotSteps - 1)) == kSlotSteps - 1;
+#pragma unroll
+        for (int kk = 0; kk < kSlabs; ++kk) {
+          if (kk % kRoundSlabs == 0 && opens) {
+            if (!ptx::MbarWaitHot(&free[d], d_phase)) {
+              ok = false;
+              break;
+            }
+            ptx::TcFenceAfter();
+          }
+          const std::uint32_t dots = tmem_half + (d * kRoundBlocks + kk % kRoundSlabs / SPB) * kHalf;
+          const bool first = kk % SPB == 0 && opens;
+          if constexpr (kBiased) {
+            if (first) {
+              UmmaI8(dots, desc_bias, desc_bias, p.idesc, 0u);
+            }
+          }
+          UmmaI8(dots, desc_w + kk * (kSlabK >> 4), desc_a + kk * (kSlabK >> 4), p.idesc, kBiased || !first ? 1u : 0u);
+          if ((kk % kRoundSlabs == kRoundSlabs - 1 || kk == kSlabs - 1) && closes) {
+            ptx::UmmaCommit(&full[d]);
+            if (++d == kRoundBuffers) {
+              d = 0;
+              d_phase ^= 1u;
+            }
+          }
+        }
+        if (!ok) {
+          break;
+        }
+        ptx::UmmaCommit(&empty[s]);
+        if constexpr (BITS == 4) {
+          ptx::UmmaCommit(&w_empty[w]);
+        }
+        if (++s == kStages) {
+          s = 0;
+        }
+        if (++w == kLanded) {
+          w = 0;
+          w_phase ^= 1u;
+        }
+      }
+      if (!ok) {
+        ReportStatus(p.status, kDeviceTimeoutMmaBarrier);
+        *abort_flag = 1;
+      }
+    } else if (warp == 3) {
+      // ------------------------------- scales (and 8-bit zero points) of the 128 weight rows -------------------------------
+      // Four blocks of every row per slot. Read by the scaling lanes themselves, one round ahead, they cost 13 of 92 us
+      // (M = 512, N = K = 4096, blocks of 32).
+      const int blocks = (slot_end - slot_begin) * kEntries;
+      const bool vector = p.vector_scales != 0 && (b_begin & 3) == 0;
+      int q = 0;
+      std::uint32_t phase = 1;
+#pragma unroll 1
+      for (int b = 0; b < blocks; b += 4) {
+        float4 scale[4];
+        [[maybe_unused]] float4 zero[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const std::int64_t row = static_cast<std::int64_t>(n0) + lane + 32 * i;
+          const std::int64_t safe = row < p.w.n ? row : 0;
+          const float *src = p.w.scales + safe * p.w.n_blocks;
+          const int first = b_begin + b;
+          if (vector && first < p.w.n_blocks) {
+            scale[i] = __ldg(reinterpret_cast<const float4 *>(src + first));
+          } else {
+            scale[i].x = first < p.w.n_blocks ? __ldg(src + first) : 0.0f;
+            scale[i].y = first + 1 < p.w.n_blocks ? __ldg(src + first + 1) : 0.0f;
+            scale[i].z = first + 2 < p.w.n_blocks ? __ldg(src + first + 2) : 0.0f;
+            scale[i].w = first + 3 < p.w.n_blocks ? __ldg(src + first + 3) : 0.0f;
+          }
+          if constexpr (BITS == 8) {
+            auto zero_point = [&](int block) {
+              return p.w.zp != nullptr && block < p.w.n_blocks ? -static_cast<float>(__ldg(p.w.zp + safe * p.w.zp_row_bytes + block)) : -128.0f;
+            };
+            zero[i] = make_float4(zero_point(first), zero_point(first + 1), zero_point(first + 2), zero_point(first + 3));
+          }
+        }
+        if (!ptx::MbarWaitHot(&t_empty[q], phase)) {
+          ReportStatus(p.status, kDeviceTimeoutEmptyBarrier);
+          *abort_flag = 1;
+          break;
+        }
+        float4 *dst = reinterpret_cast<float4 *>(weight_slots + q * Smem::kWeightSlot) + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          dst[32 * i] = scale[i];
+          if constexpr (BITS == 8) {
+            dst[kRows + 32 * i] = zero[i];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) {
+          ptx::MbarArrive(&t_full[q]);
+        }
+        if (++q == kWeightSlots) {
+          q = 0;
+          phase ^= 1u;
+        }
+      }
+    } else if (warp >= 4 && BITS == 4) {
+      // ------------------------------- 4-bit codes to signed bytes -------------------------------
+      // A thread takes one 16-byte piece (32 k, inside one block) of four rows: eight lanes of a load read
+      // 128 consecutive bytes, eight lanes of a store hit the eight bank groups through the swizzle.
+      const int t = tid - 128;
+      const int piece = t & 3;
+      const int row0 = t >> 2;             // rows row0 + 32 i
+      const int last_block = p.w.n_blocks - 1;
+      const std::uint8_t *zp_row[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const std::int64_t row = static_cast<std::int64_t>(n0) + row0 + 32 * i;
+        zp_row[i] = p.w.zp != nullptr ? p.w.zp + (row < p.w.n ? row : 0) * p.w.zp_row_bytes : nullptr;
+      }
+      auto block_of = [&](int ks) {
+        const int block = ((step0 + ks) * kSlabs + piece) / SPB;
+        return block < last_block ? block : last_block;
+      };
+      int zp_raw[4] = {0x88, 0x88, 0x88, 0x88};
+      auto fetch_zero_points = [&](int ks) {
+        if (p.w.zp != nullptr) {
+          const int byte = block_of(ks) >> 1;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            zp_raw[i] = __ldg(zp_row[i] + byte);
+          }
+        }
+      };
+      fetch_zero_points(0);
+      for (int ks = 0; ks < steps; ++ks) {
+        const int s = ks % kStages;
+        const int buffer = ks % kBuffers;
+        const int shift = (block_of(ks) & 1) * 4;
+        std::uint32_t zps[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          zps[i] = static_cast<std::uint32_t>((zp_raw[i] >> shift) & 0x0f) * 0x01010101u;
+        }
+        if (ks + 1 < steps) {
+          fetch_zero_points(ks + 1);   // used a step later: the latency of the load is not in the chain
+        }
+        if (!ptx::MbarWaitHot(&full_tma[s], static_cast<std::uint32_t>(ks / kStages) & 1u) ||
+            !ptx::MbarWaitHot(&w_empty[buffer], (static_cast<std::uint32_t>(ks / kBuffers) & 1u) ^ 1u)) {
+          ReportStatus(p.status, kDeviceTimeoutFullBarrier);
+          *abort_flag = 1;
+          break;
+        }
+        const unsigned char *packed = ring_p + s * Smem::kStageP + row0 * Smem::kRowP + piece * 16;
+        unsigned char *tile = buf_w + buffer * Smem::kBufferW + row0 * kStepK;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint4 w = *reinterpret_cast<const uint4 *>(packed + i * 32 * Smem::kRowP);
+          uint4 lo, hi;
+          lo.x = SignedCodes(w.x, zps[i]);
+          lo.y = SignedCodes(w.x >> 4, zps[i]);
+          lo.z = SignedCodes(w.y, zps[i]);
+          lo.w = SignedCodes(w.y >> 4, zps[i]);
+          hi.x = SignedCodes(w.z, zps[i]);
+          hi.y = SignedCodes(w.z >> 4, zps[i]);
+          hi.z = SignedCodes(w.w, zps[i]);
+          hi.w = SignedCodes(w.w >> 4, zps[i]);
+          unsigned char *row = tile + i * 32 * kStepK;
+          // 16-byte chunk c of a row sits at c ^ (row & 7); the four rows of a thread agree in row & 7
+          *reinterpret_cast<uint4 *>(row + (((2 * piece) ^ (row0 & 7)) << 4)) = lo;
+          *reinterpret_cast<uint4 *>(row + (((2 * piece + 1) ^ (row0 & 7)) << 4)) = hi;
+        }
+        ptx::FenceProxyAsyncShared();
+        __syncwarp();
+        if (lane == 0) {
+          ptx::MbarArrive(&w_full[buffer]);
+        }
+      }
+    }
+  } else {
+    // ------------------------------- scaling -------------------------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kHighRegs));
+    constexpr int kChunk = kHalf < 32 ? kHalf : 32;  // columns of a TMEM load
+    constexpr int kChunks = kHalf / kChunk;
+    constexpr int kGroups = kChunk / 8;              // 8-column groups of a load: 4 registers each
+    constexpr int kCells = kChunks * 4 * kGroups;    // pairs of sums a thread holds
+    const int half = (warp - 8) >> 2;
+    std::uint64_t *full = d_full + half * kDotBuffers;
+    std::uint64_t *free = d_empty + half * kDotBuffers;
+    const int quarter = warp & 3;
+    const int token0 = half * kHalf;
+    const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + half * kDotBuffers * kHalf;
+    const int row_of_lane = quarter * 32 + (lane >> 2);  // rows + 0, 8, 16, 24
+    const int pair = (lane & 3) * 2;                     // columns pair, pair + 1 of every group
+    std::uint64_t acc[kChunks][2][kGroups][2];     // [columns][upper / lower 16 rows][group][row + 0 / + 8]
+    std::uint64_t *total = totals + (tid - 256);   // this thread's own cells, kScaleWarps * 32 apart
+#pragma unroll
+    for (int i = 0; i < kCells; ++i) {
+      acc[i / (4 * kGroups)][i / (2 * kGroups) % 2][i / 2 % kGroups][i % 2] = 0;
+      total[kScaleWarps * 32 * i] = 0;
+    }
+    bool ok = true;
+    int entry = 0;
+    int slot = 0;
+    std::uint32_t slot_phase = 0;
+    int four = 0;              // block inside the slot of weight scales
+    int weight_slot = 0;
+    std::uint32_t weight_phase = 0;
+    int d = 0;
+    std::uint32_t d_phase = 0;
+    int run = 0;   // blocks since the last flush
+    constexpr float kUnit = kBiased ? 0x1p22f : 1.0f;   // what a run's sum is counted in
+    // the round's dots and scales are there; its first load is under way when this returns
+    std::uint32_t v[2][kGroups * 4];
+    auto open_round = [&]() {
+      if ((four == 0 && !ptx::MbarWaitHot(&t_full[weight_slot], weight_phase)) ||
+          (entry == 0 && !ptx::MbarWaitHot(&s_full[slot], slot_phase)) || !ptx::MbarWaitHot(&full[d], d_phase)) {
+        ReportStatus(p.status, kDeviceTimeoutEpilogueBarrier);
+        *abort_flag = 1;
+        return false;
+      }
+      ptx::TcFenceAfter();
+      TmemLoadRows(lane_base + d * kRoundBlocks * kHalf, v[0]);
+      return true;
+    };
+    ok = open_round();
+#pragma unroll 1
+    for (int round = 0; round < rounds && ok; ++round) {
+      const float *table = reinterpret_cast<const float *>(slots + slot * Smem::kSlot) + entry * Smem::kSums * BT + token0 + pair;
+      const std::uint32_t taddr = lane_base + d * kRoundBlocks * kHalf;
+      const float *weight_row = reinterpret_cast<const float *>(weight_slots + weight_slot * Smem::kWeightSlot) +
+                                row_of_lane * 4 + four;
+      float scale_now[4][kRoundBlocks];
+      [[maybe_unused]] float zero_now[4][kRoundBlocks];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        LoadRun(weight_row + 32 * r, scale_now[r]);
+        if constexpr (BITS == 8) {
+          LoadRun(weight_row + kRows * 4 + 32 * r, zero_now[r]);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < kRoundBlocks; ++e) {
+        std::uint64_t scale[4];
+        [[maybe_unused]] std::uint64_t minus_zp[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          scale[r] = Pair(scale_now[r][e], scale_now[r][e]);
+          if constexpr (BITS == 8) {
+            minus_zp[r] = Pair(zero_now[r][e], zero_now[r][e]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+        std::uint64_t sa[kGroups];
+        [[maybe_unused]] std::uint64_t sums[kGroups];
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) {
+          sa[g] = *reinterpret_cast<const std::uint64_t *>(table + e * Smem::kSums * BT + c * kChunk + 8 * g);
+          if constexpr (BITS == 8) {
+            sums[g] = *reinterpret_cast<const std::uint64_t *>(table + (e * Smem::kSums + 1) * BT + c * kChunk + 8 * g);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          TmemWaitRows(v[h]);
+          // the next load is in flight while this one is scaled
+          if (h == 0) {
+            TmemLoadRows(taddr + (16u << 16) + e * kHalf + c * kChunk, v[1]);
+          } else if (c + 1 < kChunks) {
+            TmemLoadRows(taddr + e * kHalf + (c + 1) * kChunk, v[0]);
+          } else if (e + 1 < kRoundBlocks) {
+            TmemLoadRows(taddr + (e + 1) * kHalf, v[0]);
+          } else {
+            // all dots of this round are in registers and its scales too: both may be overwritten
+            ptx::TcFenceBefore();
+            __syncwarp();
+            entry += kRoundBlocks;
+            four += kRoundBlocks;
+            const bool slot_done = entry >= kEntries;
+            const bool four_done = four >= 4;
+            if (lane == 0) {
+              ptx::MbarArrive(&free[d]);
+              if (slot_done) {
+                ptx::MbarArrive(&s_empty[slot]);
+              }
+              if (four_done) {
+                ptx::MbarArrive(&t_empty[weight_slot]);
+              }
+            }
+            if (four_done) {
+              four = 0;
+              if (++weight_slot == kWeightSlots) {
+                weight_slot = 0;
+                weight_phase ^= 1u;
+              }
+            }
+            if (slot_done) {
+              entry = 0;
+              if (++slot == kScaleSlots) {
+                slot = 0;
+                slot_phase ^= 1u;
+              }
+            }
+            if (++d == kRoundBuffers) {
+              d = 0;
+              d_phase ^= 1u;
+            }
+            if (kRoundBuffers > 1 && round + 1 < rounds) {
+              ok = open_round();
+            }
+          }
+#pragma unroll
+          for (int g = 0; g < kGroups; ++g) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              std::uint64_t dot;
+              if constexpr (kBiased) {
+                // the bits of a non-negative integer below 2^23 are those of the subnormal float dot * 2^-149: one
+                // multiply-add makes it dot * 2^-22 without the bias, exactly
+                dot = Fma2(Pair(__uint_as_float(v[h][4 * g + 2 * r]), __uint_as_float(v[h][4 * g + 2 * r + 1])),
+                           Pair(0x1p127f, 0x1p127f), Pair(-kBias * 0x1p-22f, -kBias * 0x1p-22f));
+              } else {
+                dot = Fma2(minus_zp[2 * h + r], sums[g],   // integers below 2^24: exact
+                           Pair(__int2float_rn(static_cast<int>(v[h][4 * g + 2 * r])),
+                                __int2float_rn(static_cast<int>(v[h][4 * g + 2 * r + 1]))));
+              }
+              acc[c][h][g][r] = Fma2(dot, Mul2(sa[g], scale[2 * h + r]), acc[c][h][g][r]);
+            }
+          }
+        }
+        }
+      }
+      // with one buffer the next round cannot be complete yet: the last piece was scaled first
+      if (kRoundBuffers == 1 && round + 1 < rounds) {
+        ok = open_round();
+      }
+      run += kRoundBlocks;
+      if (run == kFlushBlocks || round == rounds - 1) {
+        run = 0;
+#pragma unroll
+        for (int i = 0; i < kCells; ++i) {
+          std::uint64_t &sum = acc[i / (4 * kGroups)][i / (2 * kGroups) % 2][i / 2 % kGroups][i % 2];
+          total[kScaleWarps * 32 * i] = Fma2(sum, Pair(kUnit, kUnit), total[kScaleWarps * 32 * i]);
+          sum = 0;
+        }
+      }
+    }
+    if (ok && *abort_flag == 0) {
+      const bool whole = p.partial == nullptr; // otherwise the sum kernel adds the bias
+      float *base = whole ? p.out.y + p.out.col_offset
+                          : p.partial + static_cast<std::int64_t>(part) * p.m_total * p.w.n;
+      const std::int64_t ld = whole ? p.out.ld : p.w.n;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const std::int64_t col = static_cast<std::int64_t>(n0) + row_of_lane + 16 * h + 8 * r;
+          if (col >= p.w.n) {
+            continue;
+          }
+          const float bias = whole && p.w.bias != nullptr ? __ldg(p.w.bias + col) : 0.0f;
+#pragma unroll
+          for (int i = 0; i < kChunks * kGroups; ++i) {
+            const int c = i / kGroups, g = i % kGroups;
+            const float2 y = Unpair(total[kScaleWarps * 32 * (((c * 2 + h) * kGroups + g) * 2 + r)]);
+            const int m = m0 + token0 + c * kChunk + 8 * g + pair;
+            if (m < p.m_total) {
+              base[static_cast<std::int64_t>(m) * ld + col] = y.x + bias;
+            }
+            if (m + 1 < p.m_total) {
+              base[static_cast<std::int64_t>(m + 1) * ld + col] = y.y + bias;
+            }
+          }
+        }
+      }
+    }
+  }
+
+  ptx::TcFenceBefore();
+  __syncthreads();
+  if (warp == 0) {
+    ptx::TcFenceAfter();
+    ptx::TmemDealloc(tmem_base, kTmemColumns);
+  }
+}
+
+// ---- host side -----------------------------------------------------------------------------
+
+std::int64_t RoundUp(std::int64_t v, std::int64_t of) { return (v + of - 1) / of * of; }
+
+struct I8Layout {
+  int k_pad;       // codes of a token row
+  int m_pad;       // scales of a block
+  int blocks_pad;
+  std::size_t codes_bytes;
+  int table_rows;  // scales of the blocks; with 8-bit weights a row of sums behind each
+  std::size_t table_bytes;
+};
+
+I8Layout LayoutOf(const WeightView &w, std::int64_t m) {
+  I8Layout l{};
+  l.k_pad = static_cast<int>(RoundUp(static_cast<std::int64_t>(w.n_blocks) * w.block_size, kStepK));
+  l.m_pad = static_cast<int>(RoundUp(m, 128));
+  l.blocks_pad = l.k_pad / w.block_size;
+  l.codes_bytes = static_cast<std::size_t>(RoundUp(m * l.k_pad, 256));
+  l.table_rows = l.blocks_pad * (w.bits == 8 ? 2 : 1);
+  l.table_bytes = static_cast<std::size_t>(l.table_rows) * l.m_pad * sizeof(float);
+  return l;
+}
+
+// Tokens per CTA and the number of parts K is shared between.
+struct I8Plan {
+  int tokens;
+  int parts;
+};
+
+// A cost model in microseconds, fitted to N = K = 4096 (M = 64 ... 2048, all block sizes): a 128-k step of a tile costs
+// 0.45 for its barriers plus, per token, 0.0031 (8-bit weights: 0.0045) for every block that ends in it; a tile 8 for
+// set-up, the first copies and its stores; the partial products of a shared K cross L2 once more on their way into Y.
+I8Plan PlanOf(const WeightView &w, std::int64_t m, int sms) {
+  const std::int64_t row_tiles = (w.n + kRows - 1) / kRows;
+  const std::int64_t step_blocks = w.block_size < kStepK ? kStepK / w.block_size : 1;
+  const std::int64_t slots = (w.n_blocks + step_blocks - 1) / step_blocks;       // smallest unit of a shared K
+  const double slot_steps = w.block_size > kStepK ? static_cast<double>(w.block_size / kStepK) : 1.0;
+  const double scaling = (w.bits == 4 ? 0.0031 : 0.0045) * static_cast<double>(step_blocks);
+  I8Plan best{128, 1};
+  double best_cost = -1.0;
+  for (int parts = 1; parts <= 8; parts *= 2) {
+    if (parts > 1 && slots / parts < 4) {
+      break;
+    }
+    for (int tokens = 128; tokens >= 32; tokens /= 2) {
+      const std::int64_t tiles = row_tiles * ((m + tokens - 1) / tokens) * parts;
+      const double rounds = static_cast<double>((tiles + sms - 1) / sms);
+      double cost = rounds * (8.0 + static_cast<double>((slots + parts - 1) / parts) * slot_steps * (0.45 + scaling * tokens));
+      if (parts > 1) {
+        cost += 3.0 + static_cast<double>(parts + 1) * static_cast<double>(m) * static_cast<double>(w.n) * 4.0 / 4.0e6;
+      }
+      if (best_cost < 0.0 || cost < best_cost) {
+        best_cost = cost;
+        best = I8Plan{tokens, parts};
+      }
+    }
+  }
+  return best;
+}
+
+template <typename Kernel, typename... Args>
+bool LaunchDependent(Kernel kernel, dim3 grid, dim3 block, std::size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  if (cudaLaunchKernelEx(&config, kernel, args...) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  CountLaunch();
+  return true;
+}
+
+template <int BT, int BITS, int SPB>
+bool LaunchTile(const WeightView &w, std::int64_t m, const I8Layout &l, const std::int8_t *codes, const float *table, I8Params p,
+                int parts, cudaStream_t stream) {
+  using Smem = I8Smem<BT, BITS>;
+  CUtensorMap map_a, map_p, map_s;
+  if (!EncodeMap2D(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes, static_cast<std::uint64_t>(l.k_pad),
+                   static_cast<std::uint64_t>(m), static_cast<std::uint64_t>(l.k_pad), kStepK, BT,
+                   CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !EncodeMap2D(&map_p, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w.b, static_cast<std::uint64_t>(w.row_bytes),
+                   static_cast<std::uint64_t>(w.n), static_cast<std::uint64_t>(w.row_bytes), Smem::kRowP, kRows,
+                   BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !EncodeMap2D(&map_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, table, static_cast<std::uint64_t>(l.m_pad),
+                   static_cast<std::uint64_t>(l.table_rows), static_cast<std::uint64_t>(l.m_pad) * 4, BT,
+                   static_cast<std::uint32_t>((SPB < 4 ? 4 / SPB : 1) * Smem::kSums), CU_TENSOR_MAP_SWIZZLE_NONE)) {
+    return false;
+  }
+  auto kernel = nbits_gemm_i8_tcgen05_kernel<BT, BITS, SPB>;
+  // the register move needs exactly this many registers at launch: with fewer the second warpgroups would wait
+  // for registers that nobody gives up
+  cudaFuncAttributes attributes{};
+  if (cudaFuncGetAttributes(&attributes, kernel) != cudaSuccess ||
+      attributes.numRegs * kThreads < 256 * kLowRegs + kScaleWarps * 32 * kHighRegs ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal) != cudaSuccess) {
+    return false;
+  }
+  // kind::i8: c_format [4,6) = 2 (s32), a_format [7,10) = 1 (s8) or 0 (u8), b_format [10,13) = 1 (s8)
+  p.idesc = (2u << 4) | ((BITS == 4 ? 1u : 0u) << 7) | (1u << 10) | (static_cast<std::uint32_t>(BT / 2 >> 3) << 17) |
+            (static_cast<std::uint32_t>(kRows >> 4) << 24);
+  const dim3 grid(static_cast<unsigned>((w.n + kRows - 1) / kRows), static_cast<unsigned>((m + BT - 1) / BT),
+                  static_cast<unsigned>(parts));
+  return LaunchDependent(kernel, grid, dim3(kThreads), Smem::kTotal, stream, map_a, map_p, map_s, p);
+}
+
+template <int BT, int BITS>
+bool LaunchBlocks(const WeightView &w, std::int64_t m, const I8Layout &l, const std::int8_t *codes, const float *table,
+                  const I8Params &p, const I8Plan &plan, cudaStream_t stream) {
+  switch (w.block_size) {
+  case 32:
+    return LaunchTile<BT, BITS, 1>(w, m, l, codes, table, p, plan.parts, stream);
+  case 64:
+    return LaunchTile<BT, BITS, 2>(w, m, l, codes, table, p, plan.parts, stream);
+  case 128:
+    return LaunchTile<BT, BITS, 4>(w, m, l, codes, table, p, plan.parts, stream);
+  default:
+    return LaunchTile<BT, BITS, 8>(w, m, l, codes, table, p, plan.parts, stream);
+  }
+}
+
+template <int BITS>
+bool LaunchTiles(const WeightView &w, std::int64_t m, const I8Layout &l, const std::int8_t *codes, const float *table,
+                 const I8Params &p, const I8Plan &plan, cudaStream_t stream) {
+  switch (plan.tokens) {
+  case 128:
+    return LaunchBlocks<128, BITS>(w, m, l, codes, table, p, plan, stream);
+  case 64:
+    return LaunchBlocks<64, BITS>(w, m, l, codes, table, p, plan, stream);
+  default:
+    return LaunchBlocks<32, BITS>(w, m, l, codes, table, p, plan, stream);
+  }
+}
+
+} // namespace
+
+bool GemmI8Supports(const WeightView &w, std::int64_t m) {
+  return m > 16 && m <= (1 << 24) && w.n >= kRows && (w.bits == 4 || w.bits == 8) && w.block_size >= 32 && w.block_size <= 256 &&
+         w.k % 8 == 0 && w.k <= (1 << 24) && (w.row_bytes % 16) == 0 &&
+         (reinterpret_cast<std::uintptr_t>(w.b) & 15u) == 0 && GetEncodeTiled() != nullptr;
+}
+
+// codes [m, k_pad], scale table [rows, m_pad], partial products [parts, m, n].
+std::size_t GemmI8ScratchBytes(const WeightView &w, std::int64_t m, int sm_count) {
+  const I8Layout l = LayoutOf(w, m);
+  std::size_t bytes = l.codes_bytes + l.table_bytes;
+  const I8Plan plan = PlanOf(w, m, sm_count > 0 ? sm_count : 148);
+  if (plan.parts > 1) {
+    bytes += static_cast<std::size_t>(plan.parts) * static_cast<std::size_t>(m) * static_cast<std::size_t>(w.n) * sizeof(float);
+  }
+  return bytes;
+}
+
+const char *LaunchGemmI8(const WeightView *nodes, const OutputView *outs, int count, const float *a, std::int64_t m,
+                         unsigned char *scratch, int *status_word, cudaStream_t stream, int sm_count) {
+  if ((reinterpret_cast<std::uintptr_t>(a) & 15u) != 0) {
+    return nullptr;
+  }
+  const WeightView &first = nodes[0];
+  for (int i = 0; i < count; ++i) {
+    // the nodes read the same codes: same order of k, same blocks
+    if (!GemmI8Supports(nodes[i], m) || nodes[i].k != first.k || nodes[i].bits != first.bits ||
+        nodes[i].block_size != first.block_size) {
+      return nullptr;
+    }
+  }
+  const int sms = sm_count > 0 ? sm_count : 148;
+  const I8Layout l = LayoutOf(first, m);
+  std::int8_t *codes = reinterpret_cast<std::int8_t *>(scratch);
+  float *table = reinterpret_cast<float *>(scratch + l.codes_bytes);
+  float *partial = reinterpret_cast<float *>(scratch + l.codes_bytes + l.table_bytes);
+  const std::int64_t threads = m * (l.k_pad / 8);
+  const dim3 quantize_grid(static_cast<unsigned>((threads + 255) / 256));
+  auto quantize = first.bits == 4 ? nbits_quantize_a_i8_kernel<true> : nbits_quantize_a_i8_kernel<false>;
+  if (!LaunchDependent(quantize, quantize_grid, dim3(256), 0, stream, a, static_cast<int>(m), first.k, l.k_pad,
+                       first.block_size, l.m_pad, codes, table)) {
+    return nullptr;
+  }
+  for (int i = 0; i < count; ++i) {
+    const WeightView &w = nodes[i];
+    const I8Plan plan = PlanOf(w, m, sms);
+    I8Params p{};
+    p.w = w;
+    p.out = outs[i];
+    p.m_total = static_cast<int>(m);
+    p.status = status_word;
+    p.vector_scales = w.n_blocks % 4 == 0 && (reinterpret_cast<std::uintptr_t>(w.scales) & 15u) == 0 ? 1 : 0;
+    p.partial = plan.parts > 1 ? partial : nullptr;
+    const bool launched = w.bits == 4 ? LaunchTiles<4>(w, m, l, codes, table, p, plan, stream)
+                                      : LaunchTiles<8>(w, m, l, codes, table, p, plan, stream);
+    if (!launched || (plan.parts > 1 && !LaunchSplitKSum(partial, plan.parts, m, w, outs[i], stream, sms))) {
+      return nullptr;
+    }
+  }
+  return "nbits_gemm_i8_tcgen05_kernel";
+}
+
+} // namespace mnb

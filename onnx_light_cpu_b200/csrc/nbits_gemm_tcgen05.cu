@@ -972,14 +972,9 @@ const char *LaunchPairBits(const WeightView &w, std::int64_t m, const std::uint1
   }
   CountLaunch();
   if (plan.parts > 1) {
-    const std::int64_t total = m * w.n;
-    std::int64_t blocks = (total + 255) / 256;
-    blocks = blocks > static_cast<std::int64_t>(sms) * 8 ? static_cast<std::int64_t>(sms) * 8 : blocks;
-    if (!LaunchDependent(nbits_split_k_sum_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream,
-                         static_cast<const float *>(partial), plan.parts, m, w.n, w.bias, out)) {
+    if (!LaunchSplitKSum(partial, plan.parts, m, w, out, stream, sms)) {
       return nullptr;
     }
-    CountLaunch();
     return "nbits_gemm_tcgen05_pair_kernel(split-k)";
   }
   return "nbits_gemm_tcgen05_pair_kernel";
@@ -994,6 +989,18 @@ const char *LaunchPair(const WeightView &w, std::int64_t m, const std::uint16_t 
 std::size_t AlignScratch(std::size_t v) { return (v + 255) & ~std::size_t{255}; }
 
 } // namespace
+
+bool LaunchSplitKSum(const float *partial, int parts, std::int64_t m, const WeightView &w, OutputView out,
+                     cudaStream_t stream, int sms) {
+  std::int64_t blocks = (m * w.n + 255) / 256;
+  blocks = blocks > static_cast<std::int64_t>(sms) * 8 ? static_cast<std::int64_t>(sms) * 8 : blocks;
+  if (!LaunchDependent(nbits_split_k_sum_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, partial, parts, m,
+                       w.n, w.bias, out)) {
+    return false;
+  }
+  CountLaunch();
+  return true;
+}
 
 // bf16 activations of one call, then (K shared between pairs only) the partial products [parts][m][n].
 std::size_t GemmTcgen05ScratchBytes(const WeightView &w, std::int64_t m, int sm_count) {

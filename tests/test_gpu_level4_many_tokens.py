@@ -1,0 +1,103 @@
+"""accuracy_level 4 with more than sixteen tokens: the tcgen05 integer GEMM against the block dots in 64 bits."""
+
+import numpy as np
+import pytest
+
+import onnx_light_cpu_b200 as pkg
+from onnx_light_cpu_b200 import _capi
+from onnx_light_cpu_b200.matmul_nbits import matmul_device_group
+from onnx_light_cpu_b200.tools import synthetic as syn
+from oracle import nbits_oracle as o
+
+pytestmark = pytest.mark.gpu
+
+KERNEL = "nbits_gemm_i8_tcgen05_kernel"
+
+
+def expected(case):
+    """Y in 64 bits and the bound of a 32-bit evaluation: a term passes two roundings of its scaling, at most sixteen
+    additions of its run and one per run, part and bias behind it, each 2^-24 of a partial sum no larger than the sum
+    of the magnitudes."""
+    aq, sa = o.quantize_a(case.a, case.k, case.block_size)
+    dots = o.int8_block_dots(aq, case.b, case.zero_points, case.n, case.k, case.bits, case.block_size).astype(np.float64)
+    blocks = dots.shape[2]
+    terms = dots * sa.astype(np.float64)[:, None, :] * case.scales.reshape(case.n, blocks).astype(np.float64)[None]
+    bias = 0.0 if case.bias is None else case.bias.astype(np.float64)
+    roundings = 2 + 16 + -(-blocks // 16) + 8 + 1
+    bound = roundings * 2.0 ** -24 * (np.abs(terms).sum(axis=2) + np.abs(bias))
+    return terms.sum(axis=2) + bias, bound
+
+
+def run(case):
+    import torch
+
+    weights = pkg.MatMulNBitsWeights(case.b, case.scales, case.zero_points, case.bias, K=case.k, N=case.n,
+                                     bits=case.bits, block_size=case.block_size)
+    y = torch.full((case.m, case.n), float("nan"), device="cuda")
+    weights.matmul_device(torch.from_numpy(case.a).cuda(), y, accuracy_level=4)
+    torch.cuda.synchronize()
+    assert weights.poll_status() == 0
+    row_bytes = -(-case.k // case.block_size) * case.block_size * case.bits // 8
+    few = case.m <= 32 or (case.m <= 64 and case.n * case.k <= 2 << 20)   # two to four passes of the sixteen-token kernel
+    if case.bits == 8 or not few or row_bytes % 128 != 0:
+        assert _capi.last_kernel() == KERNEL, _capi.last_kernel()
+    weights.close()
+    return y.cpu().numpy()
+
+
+# every block size and both widths at the edges of the token tiles (32, 64, 128) and row tiles (128), an odd number of
+# blocks (last step of 128 k partly filled), K ending inside a block, more blocks than one run of sums, K shared
+# between CTAs, a column count that is odd
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("m,k,n,bs,zp,bias", [
+    (17, 1024, 128, 32, False, False), (32, 1056, 129, 32, True, True), (33, 1000, 200, 32, True, False),
+    (64, 2048, 255, 64, True, True), (65, 1088, 256, 64, False, True), (17, 1056, 200, 32, True, True), (128, 1024, 384, 128, True, True),
+    (129, 4096, 130, 32, True, False), (257, 1152, 515, 128, False, True), (40, 8192, 512, 32, True, True),
+    (100, 2304, 131, 256, True, True), (48, 14336, 640, 128, True, False), (300, 1032, 1001, 32, True, True),
+])
+def test_many_tokens_match_block_dots(cuda_device, bits, m, k, n, bs, zp, bias):
+    case = syn.make_case("lvl4many", m, k, n, bits, bs, seed=m + n + bs, zero_points=zp, bias=bias)
+    y, (ref, bound) = run(case), expected(case)
+    assert (np.abs(y - ref) <= bound).all(), float((np.abs(y - ref) / bound).max())
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_many_tokens_extreme_codes(cuda_device, bits):
+    """The largest dots either width can make: every code and zero point at an end of its range, every activation at
+    its block's maximum, and the values that have no int8 form."""
+    case = syn.make_case("lvl4ends", 70, 1024, 256, bits, 256, seed=3, zero_points=True, bias=False)
+    case.b[:] = 0xFF
+    case.b[::2] = 0
+    case.zero_points[:] = 0
+    case.zero_points[::2] = 0xFF
+    case.a[:] = 1.5
+    case.a[::2] = -1.5
+    case.a[4] = 0.0
+    y, (ref, bound) = run(case), expected(case)
+    assert (np.abs(y - ref) <= bound).all()
+    case.a[7, 300] = np.inf
+    case.a[9, 5] = np.nan
+    y = run(case)
+    assert np.isnan(y[[7, 9]]).all()
+    keep = [i for i in range(70) if i not in (7, 9)]
+    assert (np.abs(y - ref)[keep] <= bound[keep]).all()
+
+
+def test_many_tokens_group_is_the_nodes(cuda_device):
+    """Sibling nodes behind one quantization give what separate calls give; a strided output window too."""
+    import torch
+
+    cases = [syn.make_case(f"lvl4g{n}", 80, 2048, n, 4, 32, seed=n, zero_points=zp) for n, zp in ((512, False), (256, True), (131, False))]
+    nodes = [pkg.MatMulNBitsWeights(c.b, c.scales, c.zero_points, c.bias, K=c.k, N=c.n, bits=4, block_size=32) for c in cases]
+    a = torch.from_numpy(cases[0].a).cuda()
+    ys = [torch.full((80, c.n), float("nan"), device="cuda") for c in cases]
+    matmul_device_group(nodes, a, ys, accuracy_level=4)
+    assert _capi.last_kernel() == KERNEL
+    wide = torch.zeros((80, 1024), device="cuda")
+    for node, y, case in zip(nodes, ys, cases):
+        single = torch.empty_like(y)
+        node.matmul_device(a, single, accuracy_level=4)
+        assert torch.equal(single, y)
+        node.matmul_device(a, wide, accuracy_level=4, ld_y=1024, col_offset=7)
+        assert torch.equal(wide[:, 7:7 + case.n], y)
+        assert node.poll_status() == 0
