@@ -89,6 +89,10 @@ struct mnb_weights {
   float *y_dev = nullptr;
   std::size_t a_dev_bytes = 0;
   std::size_t y_dev_bytes = 0;
+  // page-locked staging of small pageable host buffers: A, then Y (host address and device alias)
+  unsigned char *stage_host = nullptr;
+  unsigned char *stage_dev = nullptr;
+  std::size_t stage_bytes = 0;
   cudaStream_t stream = nullptr;
   // last (A, Y) pair of the device-pointer entry points whose location has been checked
   const void *checked_a = nullptr;
@@ -224,6 +228,34 @@ int Grow(void **ptr, std::size_t *have, std::size_t need) {
   }
   *have = need;
   return MNB_OK;
+}
+
+// Page-locked staging of at least `need` bytes; false leaves the call without it (the copies of the runtime serve then).
+bool GrowStage(mnb_weights *h, std::size_t need) {
+  if (need <= h->stage_bytes) {
+    return true;
+  }
+  if (h->stage_host != nullptr) {
+    cudaStreamSynchronize(h->stream); // a call that failed half-way may still be reading it
+    cudaFreeHost(h->stage_host);
+    h->stage_host = nullptr;
+    h->stage_bytes = 0;
+  }
+  void *host = nullptr;
+  void *dev = nullptr;
+  if (cudaHostAlloc(&host, need, cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (cudaHostGetDevicePointer(&dev, host, 0) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFreeHost(host);
+    return false;
+  }
+  h->stage_host = static_cast<unsigned char *>(host);
+  h->stage_dev = static_cast<unsigned char *>(dev);
+  h->stage_bytes = need;
+  return true;
 }
 
 // Copies a small page-locked host buffer into device memory with a kernel: a kernel behind a
@@ -846,8 +878,10 @@ int mnb_weights_destroy(mnb_weights *h) {
       cudaFree(ptr);
     }
   }
-  if (h->status_host != nullptr) {
-    cudaFreeHost(h->status_host);
+  for (void *ptr : {static_cast<void *>(h->status_host), static_cast<void *>(h->stage_host)}) {
+    if (ptr != nullptr) {
+      cudaFreeHost(ptr);
+    }
   }
   delete h;
   return MNB_OK;
@@ -1349,6 +1383,24 @@ int mnb_matmul_host(mnb_weights *h, const float *a_host, int64_t m, int accuracy
     h->host_y_bytes = y_bytes;
   }
   const float *a_alias = h->host_a_alias;
+  float *y_alias = h->host_y_alias;
+  // Small pageable buffers (an evaluator's tensors) go through page-locked staging of this node: two memcpys on the host
+  // instead of two copies by the runtime, the second of which it starts only when the product is done (one token,
+  // K = 4096, N = 14336: 70 -> 46 us a call). Larger results keep the copy engine: stores from the SMs wait on the link.
+  constexpr std::size_t kStageLimit = std::size_t{256} << 10;
+  const std::size_t a_staged = a_alias == nullptr && a_bytes <= kStageLimit ? (a_bytes + 255) & ~std::size_t{255} : 0;
+  const std::size_t y_staged = y_alias == nullptr && y_bytes <= kStageLimit ? y_bytes : 0;
+  const float *y_stage = nullptr;
+  if (a_staged + y_staged > 0 && GrowStage(h, a_staged + y_staged)) {
+    if (a_staged > 0) {
+      std::memcpy(h->stage_host, a_host, a_bytes);
+      a_alias = reinterpret_cast<const float *>(h->stage_dev);
+    }
+    if (y_staged > 0) {
+      y_stage = reinterpret_cast<const float *>(h->stage_host + a_staged);
+      y_alias = reinterpret_cast<float *>(h->stage_dev + a_staged);
+    }
+  }
   if (a_alias != nullptr) {
     const int count16 = static_cast<int>(a_bytes / 16);
     const int tail = static_cast<int>((a_bytes - static_cast<std::size_t>(count16) * 16) / sizeof(float));
@@ -1370,7 +1422,6 @@ int mnb_matmul_host(mnb_weights *h, const float *a_host, int64_t m, int accuracy
   // decode-sized result), the kernels store straight into it through its device alias, which
   // saves a copy launch per call; any other buffer gets a device staging buffer and a
   // device-to-host copy, which keeps the SMs from waiting on the host link for large results.
-  float *y_alias = h->host_y_alias;
   if (y_alias == nullptr) {
     rc = Grow(reinterpret_cast<void **>(&h->y_dev), &h->y_dev_bytes, y_bytes);
     if (rc != MNB_OK) {
@@ -1400,6 +1451,9 @@ int mnb_matmul_host(mnb_weights *h, const float *a_host, int64_t m, int accuracy
     char text[96];
     std::snprintf(text, sizeof(text), "matmulnbits_b200: device-side wait timed out (status %d).", status);
     return Fail(MNB_ERR_DEVICE_TIMEOUT, text);
+  }
+  if (y_stage != nullptr) {
+    std::memcpy(y_host, y_stage, y_bytes);
   }
   return MNB_OK;
 }

@@ -1096,3 +1096,29 @@ def test_registered_operator_notices_rewritten_weights(cuda_device):
     ref2 = o.matmul_f64(case.a, other.b, case.scales, case.zero_points, case.bias, case.n, case.k, 4, 32)
     assert rel_err(y2, ref2) <= TOL_FP32 and rel_err(y2, y1) > 1e-2
     assert np.array_equal(session.run(case.a), y2)   # unchanged weights: the cached upload is used
+
+
+def test_host_call_staging_grows_and_mixes_with_page_locked_buffers(cuda_device):
+    """Small pageable buffers go through the node's page-locked staging: more tokens than before, fewer again, either
+    side page-locked, results above the staging limit, addresses off the 16-byte grid."""
+    import torch
+
+    full = syn.make_case("stage", 48, 1024, 1501, 4, 32, seed=8, zero_points=True, bias=True)
+    weights = pkg.MatMulNBitsWeights(full.b, full.scales, full.zero_points, full.bias, K=full.k, N=full.n, bits=4,
+                                     block_size=32)
+    a_pinned = torch.from_numpy(full.a).pin_memory()
+    y_pinned = torch.empty((48, full.n)).pin_memory()
+    for m in (1, 3, 16, 2, 43, 48, 1):   # 43 rows of Y are below 256 KB, 48 above
+        y = np.full((m, full.n), np.nan, dtype=np.float32)
+        weights.matmul_host_ptr(a_pinned.data_ptr(), m, y_pinned.data_ptr())
+        expect = y_pinned.numpy()[:m].copy()
+        shifted = np.empty(m * full.k + 1, dtype=np.float32)[1:]
+        shifted[:] = full.a[:m].ravel()
+        for a_ptr in (full.a.ctypes.data, shifted.ctypes.data, a_pinned.data_ptr()):
+            y.fill(np.nan)
+            weights.matmul_host_ptr(a_ptr, m, y.ctypes.data)
+            assert np.array_equal(y, expect)
+        y_pinned.fill_(float("nan"))
+        weights.matmul_host_ptr(shifted.ctypes.data, m, y_pinned.data_ptr())
+        assert np.array_equal(y_pinned.numpy()[:m], expect)
+    weights.close()
