@@ -188,6 +188,7 @@ struct U8Params {
   int blocks_per_part;
   int steps;
   int tiles;
+  int vector_meta;      // scales and zero points of four blocks lie aligned
 };
 
 constexpr int kU8Super = 8;                              // 32-k steps per tile of weights
@@ -204,7 +205,12 @@ __global__ void __launch_bounds__(kU8Warps * 32)
   constexpr int NT = kDigits * NTOK;   // MMA column tiles
   constexpr int kCols = NT * 8;
   __shared__ __align__(16) unsigned char tiles[kU8Warps][kU8TileBytes];
-  __shared__ float meet[kU8Warps][NTOK * 4][32];
+  // scale and zero point (as a float2) of the blocks of a tile, by row; a row padded so that the eight rows a read
+  // touches lie on different banks
+  constexpr int kTileBlocks = kU8Super / SPB;
+  constexpr int kLaneBlocks = kTileBlocks >= 2 ? kTileBlocks / 2 : 1;   // two lanes a row (one, for one block)
+  __shared__ float2 metas[kU8Warps][16][kTileBlocks + 1];
+  static_assert(NTOK * 4 * 32 * sizeof(float) <= kU8TileBytes, "the parts of K meet in the warps' tiles");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -215,12 +221,10 @@ __global__ void __launch_bounds__(kU8Warps * 32)
   const bool live = tile < p.tiles;
   const std::int64_t row0 = static_cast<std::int64_t>(live ? tile : 0) * 16;
   // rows beyond N repeat the last one; their sums are not written
-  const std::int64_t r_lo = row0 + g < p.w.n ? row0 + g : p.w.n - 1;
-  const std::int64_t r_hi = row0 + g + 8 < p.w.n ? row0 + g + 8 : p.w.n - 1;
-  const float *scale_lo = p.w.scales + r_lo * p.w.n_blocks;
-  const float *scale_hi = p.w.scales + r_hi * p.w.n_blocks;
-  const std::uint8_t *zp_lo = p.w.zp != nullptr ? p.w.zp + r_lo * p.w.zp_row_bytes : nullptr;
-  const std::uint8_t *zp_hi = p.w.zp != nullptr ? p.w.zp + r_hi * p.w.zp_row_bytes : nullptr;
+  const std::int64_t meta_row = row0 + (lane >> 1) < p.w.n ? row0 + (lane >> 1) : p.w.n - 1;
+  const int meta_first = kTileBlocks >= 2 ? (lane & 1) * kLaneBlocks : 0;
+  const float *scale_row = p.w.scales + meta_row * p.w.n_blocks;
+  const std::uint8_t *zp_row = p.w.zp != nullptr ? p.w.zp + meta_row * p.w.zp_row_bytes : nullptr;
   // digits of column g of every column tile, this lane's eight k of a step
   const unsigned char *digit_lane = p.digits + g * 32 + 8 * t;
   const int *sum_lane = p.sums + 2 * t;
@@ -249,7 +253,33 @@ __global__ void __launch_bounds__(kU8Warps * 32)
   const int s_end = block_end * SPB < p.steps ? block_end * SPB : p.steps;
 
   uint4 next[kU8Super];
+  // Scales and zero points travel with the tile they belong to, requested a tile ahead. Read where a block ends they were
+  // four words per lane and block out of sixteen rows, and the first touch of each line was waited for: K = 4096, blocks of
+  // 32, M = 8 287 -> 226 us at N = 128256, 44.9 -> 35.1 at N = 16032; blocks of 128 K = 14336, N = 4096 31.0 -> 28.8.
+  float next_scale[kLaneBlocks];
+  int next_zp[kLaneBlocks];
+  auto request_meta = [&](int s_first) {
+    const int block = s_first / SPB + meta_first;
+    if (kLaneBlocks == 4 && p.vector_meta != 0 && (block & 3) == 0 && block + 4 <= block_end) {
+      const float4 f = __ldg(reinterpret_cast<const float4 *>(scale_row + block));
+      const std::uint32_t z = zp_row != nullptr ? __ldg(reinterpret_cast<const std::uint32_t *>(zp_row + block)) : 0x80808080u;
+      const float scale4[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+      for (int i = 0; i < kLaneBlocks; ++i) {
+        next_scale[i] = scale4[i & 3];
+        next_zp[i] = static_cast<int>((z >> (8 * i)) & 0xffu);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kLaneBlocks; ++i) {
+        const bool inside = block + i < block_end;
+        next_scale[i] = inside ? __ldg(scale_row + block + i) : 0.0f;
+        next_zp[i] = inside && zp_row != nullptr ? static_cast<int>(__ldg(zp_row + block + i)) : 128;
+      }
+    }
+  };
   auto request = [&](int s_first) {
+    request_meta(s_first);
     const int byte = s_first * 32 + copy_byte;
     const bool inside = byte + 16 <= s_end * 32;
 #pragma unroll
@@ -274,6 +304,12 @@ __global__ void __launch_bounds__(kU8Warps * 32)
 #pragma unroll
     for (int i = 0; i < kU8Super; ++i) {
       *reinterpret_cast<uint4 *>(my_tile + (2 * i + copy_row) * kU8TileRowBytes + copy_byte) = next[i];
+    }
+    if (kTileBlocks >= 2 || (lane & 1) == 0) {
+#pragma unroll
+      for (int i = 0; i < kLaneBlocks; ++i) {
+        metas[warp][lane >> 1][meta_first + i] = make_float2(next_scale[i], __int_as_float(next_zp[i]));
+      }
     }
     __syncwarp();
     if (s0 + kU8Super < s_end) {
@@ -314,10 +350,12 @@ __global__ void __launch_bounds__(kU8Warps * 32)
         if ((u + 1) % SPB == 0) {
           // a quantization block is complete
           const int block = s / SPB;
-          const float ws_lo = __ldg(scale_lo + block);
-          const float ws_hi = __ldg(scale_hi + block);
-          const int z_lo = zp_lo != nullptr ? static_cast<int>(__ldg(zp_lo + block)) : 128;
-          const int z_hi = zp_hi != nullptr ? static_cast<int>(__ldg(zp_hi + block)) : 128;
+          const float2 meta_lo = metas[warp][g][u / SPB];
+          const float2 meta_hi = metas[warp][g + 8][u / SPB];
+          const float ws_lo = meta_lo.x;
+          const float ws_hi = meta_hi.x;
+          const int z_lo = __float_as_int(meta_lo.y);
+          const int z_hi = __float_as_int(meta_hi.y);
           const int *sum_block = sum_lane + block * (2 * 8 * NTOK);
 #pragma unroll
           for (int j = 0; j < NTOK; ++j) {
@@ -346,12 +384,14 @@ __global__ void __launch_bounds__(kU8Warps * 32)
     }
   }
 
-  // the parts of K of a row tile meet in shared memory; the first part's warp writes the rows
+  // the parts of K of a row tile meet in shared memory, in the warps' own tiles; the first part's warp writes the rows
+  float *meet = reinterpret_cast<float *>(my_tile) + lane;
+  __syncwarp();
 #pragma unroll
   for (int j = 0; j < NTOK; ++j) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      meet[warp][j * 4 + i][lane] = acc[j][i];
+      meet[(j * 4 + i) * 32] = acc[j][i];
     }
   }
   __syncthreads();
@@ -362,7 +402,7 @@ __global__ void __launch_bounds__(kU8Warps * 32)
       for (int i = 0; i < 4; ++i) {
         float total = acc[j][i];
         for (int other = 1; other < p.parts; ++other) {
-          total += meet[warp + other][j * 4 + i][lane];
+          total += meet[other * (kU8TileBytes / 4) + (j * 4 + i) * 32];
         }
         const int token = 8 * j + 2 * t + (i & 1);
         const std::int64_t row = row0 + g + (i >> 1) * 8;
@@ -576,6 +616,27 @@ int PartsFor(const WeightView &w, int tiles, int sm_count) {
   return parts;
 }
 
+// The same for the level 0 kernel, two CTAs per SM: a vocabulary-sized node, whose tiles fill the SMs without parts of K,
+// is cut where that makes the last wave fuller (N = 128256: 1002 CTAs are 3.4 waves of 296, in halves 6.8; K = 4096,
+// blocks of 32, M = 8: 226 us whole, 204 in halves, 215 in quarters, 233 in eighths; a part costs about 2 % of a whole row).
+int PartsForDigits(const WeightView &w, int tiles, int sm_count) {
+  int best = PartsFor(w, tiles, sm_count);
+  if (best > 1) {
+    return best;
+  }
+  const std::int64_t slots = std::int64_t{2} * (sm_count > 0 ? sm_count : 148);
+  double best_cost = -1.0;
+  for (int parts = 1; parts <= 4 && w.n_blocks >= 4 * parts; parts *= 2) {
+    const std::int64_t ctas = (static_cast<std::int64_t>(tiles) * parts + kU8Warps - 1) / kU8Warps;
+    const double cost = static_cast<double>((ctas + slots - 1) / slots) * (1.0 / parts + 0.02);
+    if (best_cost < 0.0 || cost < best_cost) {
+      best_cost = cost;
+      best = parts;
+    }
+  }
+  return best;
+}
+
 template <int NTOK>
 cudaError_t LaunchU8Int8(const U8Int8Params &p, int steps_per_block, unsigned grid, cudaStream_t stream) {
   switch (steps_per_block) {
@@ -666,8 +727,12 @@ const char *LaunchGemvU8Mma(const WeightView &w, const float *a, std::int64_t m,
   p.out = out;
   p.m_total = static_cast<int>(m);
   p.steps = layout.steps;
+  p.vector_meta = w.n_blocks % 4 == 0 && (reinterpret_cast<std::uintptr_t>(w.scales) & 15u) == 0 &&
+                          (reinterpret_cast<std::uintptr_t>(w.zp) & 3u) == 0
+                      ? 1
+                      : 0;
   p.tiles = static_cast<int>((w.n + 15) / 16);
-  const int parts = PartsFor(w, p.tiles, sm_count);
+  const int parts = PartsForDigits(w, p.tiles, sm_count);
   p.parts = parts;
   p.blocks_per_part = (w.n_blocks + parts - 1) / parts;
   const int tiles_per_cta = kU8Warps / parts;

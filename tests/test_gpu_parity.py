@@ -1122,3 +1122,17 @@ def test_host_call_staging_grows_and_mixes_with_page_locked_buffers(cuda_device)
         weights.matmul_host_ptr(shifted.ctypes.data, m, y_pinned.data_ptr())
         assert np.array_equal(y_pinned.numpy()[:m], expect)
     weights.close()
+
+
+# scales and zero points requested a tile ahead: rows of blocks that can be read four at a time and rows that cannot, parts
+# of K that begin off a group of four blocks, a tile that ends early, a node wide enough to be cut for its last wave
+@pytest.mark.parametrize("m,k,n,bs,zp", [
+    (8, 1024, 200, 32, True), (8, 1056, 65, 32, True), (5, 1184, 33, 32, False), (16, 1088, 40, 64, True),
+    (9, 1152, 31, 128, True), (6, 4352, 17, 256, True), (8, 3104, 50, 32, True), (8, 1024, 50003, 32, True),
+    (6, 768, 38001, 128, False),
+])
+def test_eight_bit_digits_scales_by_tile(cuda_device, m, k, n, bs, zp):
+    case = syn.make_case("u8meta", m, k, n, 8, bs, seed=m + n, zero_points=zp, bias=True)
+    y, kernel = run_device(case)
+    assert kernel == "nbits_gemv_u8_mma_kernel", kernel
+    assert rel_err(y, oracle_f64(case)) <= TOL_FP32   # 22 bits of the row maximum: 5e-7 per product
