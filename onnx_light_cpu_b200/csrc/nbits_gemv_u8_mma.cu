@@ -195,6 +195,67 @@ constexpr int kU8Super = 8;                              // 32-k steps per tile 
 constexpr int kU8TileRowBytes = kU8Super * 32 + 32;      // 256 bytes of a row, padded: fragment reads hit 32 banks
 constexpr int kU8TileBytes = 16 * kU8TileRowBytes;
 
+// Scales and zero points of a warp's sixteen rows. They travel with the tile of weights they belong to, requested a tile
+// ahead. Read where a block ends they were four words per lane and block out of sixteen rows, and the first touch of each
+// line was waited for: level 0, K = 4096, blocks of 32, M = 8 287 -> 226 us at N = 128256, 44.9 -> 35.1 at N = 16032;
+// blocks of 128, K = 14336, N = 4096 31.0 -> 28.8.
+template <int SPB> struct TileMeta {
+  static constexpr int kTileBlocks = kU8Super / SPB;
+  static constexpr int kLaneBlocks = kTileBlocks >= 2 ? kTileBlocks / 2 : 1; // two lanes a row (one, for one block)
+  // (scale, zero point) by row and block; a row padded so that the eight rows a read touches lie on different banks
+  using Cells = float2[16][kTileBlocks + 1];
+
+  const float *scale_row;
+  const std::uint8_t *zp_row;
+  int first;      // this lane's first block of a tile
+  bool vector;    // four blocks of a row lie aligned
+  float scale[kLaneBlocks];
+  int zp[kLaneBlocks];
+
+  __device__ __forceinline__ void Init(const WeightView &w, std::int64_t row0, int lane, int vector_meta) {
+    const std::int64_t row = row0 + (lane >> 1) < w.n ? row0 + (lane >> 1) : w.n - 1;
+    scale_row = w.scales + row * w.n_blocks;
+    zp_row = w.zp != nullptr ? w.zp + row * w.zp_row_bytes : nullptr;
+    first = kTileBlocks >= 2 ? (lane & 1) * kLaneBlocks : 0;
+    vector = kLaneBlocks == 4 && vector_meta != 0;
+  }
+
+  __device__ __forceinline__ void Request(int tile_block, int block_end) {
+    const int block = tile_block + first;
+    if (vector && (block & 3) == 0 && block + 4 <= block_end) {
+      const float4 f = __ldg(reinterpret_cast<const float4 *>(scale_row + block));
+      const std::uint32_t z = zp_row != nullptr ? __ldg(reinterpret_cast<const std::uint32_t *>(zp_row + block)) : 0x80808080u;
+      const float scale4[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+      for (int i = 0; i < kLaneBlocks; ++i) {
+        scale[i] = scale4[i & 3];
+        zp[i] = static_cast<int>((z >> (8 * i)) & 0xffu);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kLaneBlocks; ++i) {
+        const bool inside = block + i < block_end;
+        scale[i] = inside ? __ldg(scale_row + block + i) : 0.0f;
+        zp[i] = inside && zp_row != nullptr ? static_cast<int>(__ldg(zp_row + block + i)) : 128;
+      }
+    }
+  }
+
+  __device__ __forceinline__ void Park(Cells &cells, int lane) const {
+    if (kTileBlocks >= 2 || (lane & 1) == 0) {
+#pragma unroll
+      for (int i = 0; i < kLaneBlocks; ++i) {
+        cells[lane >> 1][first + i] = make_float2(scale[i], __int_as_float(zp[i]));
+      }
+    }
+  }
+};
+
+bool VectorMeta(const WeightView &w) {
+  return w.n_blocks % 4 == 0 && (reinterpret_cast<std::uintptr_t>(w.scales) & 15u) == 0 &&
+         (reinterpret_cast<std::uintptr_t>(w.zp) & 3u) == 0;
+}
+
 // SPB = 32-k steps per quantization block (1, 2, 4, 8): a part of K starts on a block and tiles are eight steps,
 // so where a block starts and ends inside a tile is known at compile time (a fresh accumulator there, no
 // clearing, no test per step).
@@ -205,11 +266,7 @@ __global__ void __launch_bounds__(kU8Warps * 32)
   constexpr int NT = kDigits * NTOK;   // MMA column tiles
   constexpr int kCols = NT * 8;
   __shared__ __align__(16) unsigned char tiles[kU8Warps][kU8TileBytes];
-  // scale and zero point (as a float2) of the blocks of a tile, by row; a row padded so that the eight rows a read
-  // touches lie on different banks
-  constexpr int kTileBlocks = kU8Super / SPB;
-  constexpr int kLaneBlocks = kTileBlocks >= 2 ? kTileBlocks / 2 : 1;   // two lanes a row (one, for one block)
-  __shared__ float2 metas[kU8Warps][16][kTileBlocks + 1];
+  __shared__ typename TileMeta<SPB>::Cells metas[kU8Warps];
   static_assert(NTOK * 4 * 32 * sizeof(float) <= kU8TileBytes, "the parts of K meet in the warps' tiles");
 
   const int warp = threadIdx.x >> 5;
@@ -221,10 +278,8 @@ __global__ void __launch_bounds__(kU8Warps * 32)
   const bool live = tile < p.tiles;
   const std::int64_t row0 = static_cast<std::int64_t>(live ? tile : 0) * 16;
   // rows beyond N repeat the last one; their sums are not written
-  const std::int64_t meta_row = row0 + (lane >> 1) < p.w.n ? row0 + (lane >> 1) : p.w.n - 1;
-  const int meta_first = kTileBlocks >= 2 ? (lane & 1) * kLaneBlocks : 0;
-  const float *scale_row = p.w.scales + meta_row * p.w.n_blocks;
-  const std::uint8_t *zp_row = p.w.zp != nullptr ? p.w.zp + meta_row * p.w.zp_row_bytes : nullptr;
+  TileMeta<SPB> meta;
+  meta.Init(p.w, row0, lane, p.vector_meta);
   // digits of column g of every column tile, this lane's eight k of a step
   const unsigned char *digit_lane = p.digits + g * 32 + 8 * t;
   const int *sum_lane = p.sums + 2 * t;
@@ -253,33 +308,8 @@ __global__ void __launch_bounds__(kU8Warps * 32)
   const int s_end = block_end * SPB < p.steps ? block_end * SPB : p.steps;
 
   uint4 next[kU8Super];
-  // Scales and zero points travel with the tile they belong to, requested a tile ahead. Read where a block ends they were
-  // four words per lane and block out of sixteen rows, and the first touch of each line was waited for: K = 4096, blocks of
-  // 32, M = 8 287 -> 226 us at N = 128256, 44.9 -> 35.1 at N = 16032; blocks of 128 K = 14336, N = 4096 31.0 -> 28.8.
-  float next_scale[kLaneBlocks];
-  int next_zp[kLaneBlocks];
-  auto request_meta = [&](int s_first) {
-    const int block = s_first / SPB + meta_first;
-    if (kLaneBlocks == 4 && p.vector_meta != 0 && (block & 3) == 0 && block + 4 <= block_end) {
-      const float4 f = __ldg(reinterpret_cast<const float4 *>(scale_row + block));
-      const std::uint32_t z = zp_row != nullptr ? __ldg(reinterpret_cast<const std::uint32_t *>(zp_row + block)) : 0x80808080u;
-      const float scale4[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-      for (int i = 0; i < kLaneBlocks; ++i) {
-        next_scale[i] = scale4[i & 3];
-        next_zp[i] = static_cast<int>((z >> (8 * i)) & 0xffu);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < kLaneBlocks; ++i) {
-        const bool inside = block + i < block_end;
-        next_scale[i] = inside ? __ldg(scale_row + block + i) : 0.0f;
-        next_zp[i] = inside && zp_row != nullptr ? static_cast<int>(__ldg(zp_row + block + i)) : 128;
-      }
-    }
-  };
   auto request = [&](int s_first) {
-    request_meta(s_first);
+    meta.Request(s_first / SPB, block_end);
     const int byte = s_first * 32 + copy_byte;
     const bool inside = byte + 16 <= s_end * 32;
 #pragma unroll
@@ -305,12 +335,7 @@ __global__ void __launch_bounds__(kU8Warps * 32)
     for (int i = 0; i < kU8Super; ++i) {
       *reinterpret_cast<uint4 *>(my_tile + (2 * i + copy_row) * kU8TileRowBytes + copy_byte) = next[i];
     }
-    if (kTileBlocks >= 2 || (lane & 1) == 0) {
-#pragma unroll
-      for (int i = 0; i < kLaneBlocks; ++i) {
-        metas[warp][lane >> 1][meta_first + i] = make_float2(next_scale[i], __int_as_float(next_zp[i]));
-      }
-    }
+    meta.Park(metas[warp], lane);
     __syncwarp();
     if (s0 + kU8Super < s_end) {
       request(s0 + kU8Super);
@@ -455,6 +480,7 @@ struct U8Int8Params {
   int blocks_per_part;
   int steps;
   int tiles;
+  int vector_meta;         // scales and zero points of four blocks lie aligned
 };
 
 template <int NTOK, int SPB>
@@ -462,7 +488,8 @@ __global__ void __launch_bounds__(kU8Warps * 32)
     nbits_gemv_u8_int8_mma_kernel(const U8Int8Params p) {
   static_assert(SPB == 1 || SPB == 2 || SPB == 4 || SPB == 8, "blocks of 32 ... 256");
   __shared__ __align__(16) unsigned char tiles[kU8Warps][kU8TileBytes];
-  __shared__ float meet[kU8Warps][NTOK * 4][32];
+  __shared__ typename TileMeta<SPB>::Cells metas[kU8Warps];
+  static_assert(NTOK * 4 * 32 * sizeof(float) <= kU8TileBytes, "the parts of K meet in the warps' tiles");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -472,12 +499,8 @@ __global__ void __launch_bounds__(kU8Warps * 32)
   const int tile = blockIdx.x * (kU8Warps / p.parts) + warp / p.parts;
   const bool live = tile < p.tiles;
   const std::int64_t row0 = static_cast<std::int64_t>(live ? tile : 0) * 16;
-  const std::int64_t r_lo = row0 + g < p.w.n ? row0 + g : p.w.n - 1;
-  const std::int64_t r_hi = row0 + g + 8 < p.w.n ? row0 + g + 8 : p.w.n - 1;
-  const float *scale_lo = p.w.scales + r_lo * p.w.n_blocks;
-  const float *scale_hi = p.w.scales + r_hi * p.w.n_blocks;
-  const std::uint8_t *zp_lo = p.w.zp != nullptr ? p.w.zp + r_lo * p.w.zp_row_bytes : nullptr;
-  const std::uint8_t *zp_hi = p.w.zp != nullptr ? p.w.zp + r_hi * p.w.zp_row_bytes : nullptr;
+  TileMeta<SPB> meta;
+  meta.Init(p.w, row0, lane, p.vector_meta);
   // MMA column g of tile j is token 8 j + g; outputs of this lane are tokens 8 j + 2 t and 8 j + 2 t + 1.
   // Tokens beyond M repeat the last one; their sums are not written.
   const signed char *act_lane[NTOK];
@@ -513,6 +536,7 @@ __global__ void __launch_bounds__(kU8Warps * 32)
 
   uint4 next[kU8Super];
   auto request = [&](int s_first) {
+    meta.Request(s_first / SPB, block_end);
     const int byte = s_first * 32 + copy_byte;
     const bool inside = byte + 16 <= s_end * 32;
 #pragma unroll
@@ -536,6 +560,7 @@ __global__ void __launch_bounds__(kU8Warps * 32)
     for (int i = 0; i < kU8Super; ++i) {
       *reinterpret_cast<uint4 *>(my_tile + (2 * i + copy_row) * kU8TileRowBytes + copy_byte) = next[i];
     }
+    meta.Park(metas[warp], lane);
     __syncwarp();
     if (s0 + kU8Super < s_end) {
       request(s0 + kU8Super);
@@ -558,10 +583,12 @@ __global__ void __launch_bounds__(kU8Warps * 32)
         if ((u + 1) % SPB == 0) {
           // a quantization block is complete
           const int block = s / SPB;
-          const float ws_lo = __ldg(scale_lo + block);
-          const float ws_hi = __ldg(scale_hi + block);
-          const int z_lo = zp_lo != nullptr ? static_cast<int>(__ldg(zp_lo + block)) : 128;
-          const int z_hi = zp_hi != nullptr ? static_cast<int>(__ldg(zp_hi + block)) : 128;
+          const float2 meta_lo = metas[warp][g][u / SPB];
+          const float2 meta_hi = metas[warp][g + 8][u / SPB];
+          const float ws_lo = meta_lo.x;
+          const float ws_hi = meta_hi.x;
+          const int z_lo = __float_as_int(meta_lo.y);
+          const int z_hi = __float_as_int(meta_hi.y);
 #pragma unroll
           for (int j = 0; j < NTOK; ++j) {
             const float sa_a = __ldg(p.a_scales + token_a[j] * p.w.n_blocks + block);
@@ -578,11 +605,13 @@ __global__ void __launch_bounds__(kU8Warps * 32)
     }
   }
 
+  float *meet = reinterpret_cast<float *>(my_tile) + lane;
+  __syncwarp();
 #pragma unroll
   for (int j = 0; j < NTOK; ++j) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      meet[warp][j * 4 + i][lane] = acc[j][i];
+      meet[(j * 4 + i) * 32] = acc[j][i];
     }
   }
   __syncthreads();
@@ -593,7 +622,7 @@ __global__ void __launch_bounds__(kU8Warps * 32)
       for (int i = 0; i < 4; ++i) {
         float total = acc[j][i];
         for (int other = 1; other < p.parts; ++other) {
-          total += meet[warp + other][j * 4 + i][lane];
+          total += meet[other * (kU8TileBytes / 4) + (j * 4 + i) * 32];
         }
         const int token = 8 * j + 2 * t + (i & 1);
         const std::int64_t row = row0 + g + (i >> 1) * 8;
@@ -674,6 +703,7 @@ const char *LaunchGemvU8Int8Mma(const WeightView &w, const std::int8_t *aq, cons
   p.out = out;
   p.m_total = static_cast<int>(m);
   p.steps = w.row_bytes / 32;
+  p.vector_meta = VectorMeta(w) ? 1 : 0;
   p.tiles = static_cast<int>((w.n + 15) / 16);
   p.parts = PartsFor(w, p.tiles, sm_count);
   p.blocks_per_part = (w.n_blocks + p.parts - 1) / p.parts;
@@ -727,10 +757,7 @@ const char *LaunchGemvU8Mma(const WeightView &w, const float *a, std::int64_t m,
   p.out = out;
   p.m_total = static_cast<int>(m);
   p.steps = layout.steps;
-  p.vector_meta = w.n_blocks % 4 == 0 && (reinterpret_cast<std::uintptr_t>(w.scales) & 15u) == 0 &&
-                          (reinterpret_cast<std::uintptr_t>(w.zp) & 3u) == 0
-                      ? 1
-                      : 0;
+  p.vector_meta = VectorMeta(w) ? 1 : 0;
   p.tiles = static_cast<int>((w.n + 15) / 16);
   const int parts = PartsForDigits(w, p.tiles, sm_count);
   p.parts = parts;

@@ -1136,3 +1136,7 @@ def test_eight_bit_digits_scales_by_tile(cuda_device, m, k, n, bs, zp):
     y, kernel = run_device(case)
     assert kernel == "nbits_gemv_u8_mma_kernel", kernel
     assert rel_err(y, oracle_f64(case)) <= TOL_FP32   # 22 bits of the row maximum: 5e-7 per product
+    y, kernel = run_device(case, accuracy_level=4)
+    assert kernel == "nbits_gemv_u8_int8_mma_kernel", kernel
+    ref = o.matmul_int8(case.a, case.b, case.scales, case.zero_points, case.bias, n, k, 8, bs)
+    assert rel_err(y, ref) <= TOL_FP32   # same integers, fp32 scaling in a different order
