@@ -670,83 +670,83 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) {
-        std::uint64_t sa[kGroups];
-        [[maybe_unused]] std::uint64_t sums[kGroups];
-#pragma unroll
-        for (int g = 0; g < kGroups; ++g) {
-          sa[g] = *reinterpret_cast<const std::uint64_t *>(table + e * Smem::kSums * BT + c * kChunk + 8 * g);
-          if constexpr (BITS == 8) {
-            sums[g] = *reinterpret_cast<const std::uint64_t *>(table + (e * Smem::kSums + 1) * BT + c * kChunk + 8 * g);
-          }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          TmemWaitRows(v[h]);
-          // the next load is in flight while this one is scaled
-          if (h == 0) {
-            TmemLoadRows(taddr + (16u << 16) + e * kHalf + c * kChunk, v[1]);
-          } else if (c + 1 < kChunks) {
-            TmemLoadRows(taddr + e * kHalf + (c + 1) * kChunk, v[0]);
-          } else if (e + 1 < kRoundBlocks) {
-            TmemLoadRows(taddr + (e + 1) * kHalf, v[0]);
-          } else {
-            // all dots of this round are in registers and its scales too: both may be overwritten
-            ptx::TcFenceBefore();
-            __syncwarp();
-            entry += kRoundBlocks;
-            four += kRoundBlocks;
-            const bool slot_done = entry >= kEntries;
-            const bool four_done = four >= 4;
-            if (lane == 0) {
-              ptx::MbarArrive(&free[d]);
-              if (slot_done) {
-                ptx::MbarArrive(&s_empty[slot]);
-              }
-              if (four_done) {
-                ptx::MbarArrive(&t_empty[weight_slot]);
-              }
-            }
-            if (four_done) {
-              four = 0;
-              if (++weight_slot == kWeightSlots) {
-                weight_slot = 0;
-                weight_phase ^= 1u;
-              }
-            }
-            if (slot_done) {
-              entry = 0;
-              if (++slot == kScaleSlots) {
-                slot = 0;
-                slot_phase ^= 1u;
-              }
-            }
-            if (++d == kRoundBuffers) {
-              d = 0;
-              d_phase ^= 1u;
-            }
-            if (kRoundBuffers > 1 && round + 1 < rounds) {
-              ok = open_round();
-            }
-          }
+          std::uint64_t sa[kGroups];
+          [[maybe_unused]] std::uint64_t sums[kGroups];
 #pragma unroll
           for (int g = 0; g < kGroups; ++g) {
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              std::uint64_t dot;
-              if constexpr (kBiased) {
-                // the bits of a non-negative integer below 2^23 are those of the subnormal float dot * 2^-149: one
-                // multiply-add makes it dot * 2^-22 without the bias, exactly
-                dot = Fma2(Pair(__uint_as_float(v[h][4 * g + 2 * r]), __uint_as_float(v[h][4 * g + 2 * r + 1])),
-                           Pair(0x1p127f, 0x1p127f), Pair(-kBias * 0x1p-22f, -kBias * 0x1p-22f));
-              } else {
-                dot = Fma2(minus_zp[2 * h + r], sums[g],   // integers below 2^24: exact
-                           Pair(__int2float_rn(static_cast<int>(v[h][4 * g + 2 * r])),
-                                __int2float_rn(static_cast<int>(v[h][4 * g + 2 * r + 1]))));
-              }
-              acc[c][h][g][r] = Fma2(dot, Mul2(sa[g], scale[2 * h + r]), acc[c][h][g][r]);
+            sa[g] = *reinterpret_cast<const std::uint64_t *>(table + e * Smem::kSums * BT + c * kChunk + 8 * g);
+            if constexpr (BITS == 8) {
+              sums[g] = *reinterpret_cast<const std::uint64_t *>(table + (e * Smem::kSums + 1) * BT + c * kChunk + 8 * g);
             }
           }
-        }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            TmemWaitRows(v[h]);
+            // the next load is in flight while this one is scaled
+            if (h == 0) {
+              TmemLoadRows(taddr + (16u << 16) + e * kHalf + c * kChunk, v[1]);
+            } else if (c + 1 < kChunks) {
+              TmemLoadRows(taddr + e * kHalf + (c + 1) * kChunk, v[0]);
+            } else if (e + 1 < kRoundBlocks) {
+              TmemLoadRows(taddr + (e + 1) * kHalf, v[0]);
+            } else {
+              // all dots of this round are in registers and its scales too: both may be overwritten
+              ptx::TcFenceBefore();
+              __syncwarp();
+              entry += kRoundBlocks;
+              four += kRoundBlocks;
+              const bool slot_done = entry >= kEntries;
+              const bool four_done = four >= 4;
+              if (lane == 0) {
+                ptx::MbarArrive(&free[d]);
+                if (slot_done) {
+                  ptx::MbarArrive(&s_empty[slot]);
+                }
+                if (four_done) {
+                  ptx::MbarArrive(&t_empty[weight_slot]);
+                }
+              }
+              if (four_done) {
+                four = 0;
+                if (++weight_slot == kWeightSlots) {
+                  weight_slot = 0;
+                  weight_phase ^= 1u;
+                }
+              }
+              if (slot_done) {
+                entry = 0;
+                if (++slot == kScaleSlots) {
+                  slot = 0;
+                  slot_phase ^= 1u;
+                }
+              }
+              if (++d == kRoundBuffers) {
+                d = 0;
+                d_phase ^= 1u;
+              }
+              if (kRoundBuffers > 1 && round + 1 < rounds) {
+                ok = open_round();
+              }
+            }
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g) {
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                std::uint64_t dot;
+                if constexpr (kBiased) {
+                  // the bits of a non-negative integer below 2^23 are those of the subnormal float dot * 2^-149: one
+                  // multiply-add makes it dot * 2^-22 without the bias, exactly
+                  dot = Fma2(Pair(__uint_as_float(v[h][4 * g + 2 * r]), __uint_as_float(v[h][4 * g + 2 * r + 1])),
+                             Pair(0x1p127f, 0x1p127f), Pair(-kBias * 0x1p-22f, -kBias * 0x1p-22f));
+                } else {
+                  dot = Fma2(minus_zp[2 * h + r], sums[g],   // integers below 2^24: exact
+                             Pair(__int2float_rn(static_cast<int>(v[h][4 * g + 2 * r])),
+                                  __int2float_rn(static_cast<int>(v[h][4 * g + 2 * r + 1]))));
+                }
+                acc[c][h][g][r] = Fma2(dot, Mul2(sa[g], scale[2 * h + r]), acc[c][h][g][r]);
+              }
+            }
+          }
         }
       }
       // with one buffer the next round cannot be complete yet: the last piece was scaled first
